@@ -792,29 +792,11 @@ int pdgpu_get_forces(pdgpu_ctx *c, int32_t sys, double *f) {
     return PDGPU_ERR_ARG;
   }
   Pack &P = *e->pack;
-  int n = P.v.n_atoms;
-  std::vector<long long> a(3 * (size_t)n), h(3 * (size_t)n);
-  std::vector<double> g(3 * (size_t)n);
-  const long long *fs[3] = {P.v.fx, P.v.fy, P.v.fz};
-  const double *gs[3] = {P.v.gx, P.v.gy, P.v.gz};
-  const long long *hs[3] = {P.v.hx, P.v.hy, P.v.hz};
-  for (int k = 0; k < 3; k++) {
-    size_t o = (size_t)k * n;
-    PDGPU_CUDA(cudaMemcpyAsync(a.data() + o, fs[k], sizeof(long long) * n, cudaMemcpyDeviceToHost, c->st));
-    PDGPU_CUDA(cudaMemcpyAsync(g.data() + o, gs[k], sizeof(double) * n, cudaMemcpyDeviceToHost, c->st));
-    PDGPU_CUDA(cudaMemcpyAsync(h.data() + o, hs[k], sizeof(long long) * n, cudaMemcpyDeviceToHost, c->st));
-  }
-  int r = sync_check(c, "get_forces");
+  int r = pack_ensure_stage(&P);
   if (r) return r;
-  // the integrator's sum: fixed-point scattered terms, FP64 pair forces,
-  // fixed-point j side of the tile passes
-  double s = consts().N_per_kcalmolA;
-  for (int i = 0; i < n; i++)
-    for (int k = 0; k < 3; k++) {
-      size_t q = (size_t)k * n + i;
-      f[3 * i + k] = ((double)a[q] * kInvForceScale + g[q] + (double)h[q] * kInvJScale) * s;
-    }
-  return PDGPU_OK;
+  launch_forces_out(P.v, consts().N_per_kcalmolA, P.stage, c->st);
+  PDGPU_CUDA(cudaMemcpyAsync(f, P.stage, sizeof(double) * 3 * (size_t)P.v.n_atoms, cudaMemcpyDeviceToHost, c->st));
+  return sync_check(c, "get_forces");
 }
 
 int pdgpu_get_born_radii(pdgpu_ctx *c, int32_t sys, double *born) {
@@ -1309,19 +1291,14 @@ int pdgpu_sasa_lcpo_get(pdgpu_ctx *c, int32_t sys, double *sasa, double *deriv) 
   }
   const size_t N = (size_t)e->pack->v.n_atoms;
   if (sasa) PDGPU_CUDA(cudaMemcpyAsync(sasa, lc.sasa, sizeof(double) * N, cudaMemcpyDeviceToHost, c->st));
-  std::vector<double> d;
-  if (deriv) {
-    d.resize(3 * N);
-    PDGPU_CUDA(cudaMemcpyAsync(d.data(), lc.deriv, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, c->st));
+  if (deriv) {  // interleaved on the device, one block copied
+    Pack &P = *e->pack;
+    int r = pack_ensure_stage(&P);
+    if (r) return r;
+    launch_soa_to_aos(P.stage, lc.deriv, lc.deriv + N, lc.deriv + 2 * N, (int)N, c->st);
+    PDGPU_CUDA(cudaMemcpyAsync(deriv, P.stage, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, c->st));
   }
-  int r = sync_check(c, "sasa_lcpo_get");
-  if (r) return r;
-  for (size_t i = 0; i < N && deriv; i++) {
-    deriv[3 * i] = d[i];
-    deriv[3 * i + 1] = d[N + i];
-    deriv[3 * i + 2] = d[2 * N + i];
-  }
-  return PDGPU_OK;
+  return sync_check(c, "sasa_lcpo_get");
 }
 }  // extern "C"
 

@@ -76,6 +76,31 @@ __global__ void k_soa_to_aos(double *aos, const double *X, const double *Y, cons
   aos[3 * (size_t)i + 1] = Y[i];
   aos[3 * (size_t)i + 2] = Z[i];
 }
+// The forces of the handle in N, interleaved [n][3], as the caller gets them:
+// the integrator's sum (fixed-point scattered terms, FP64 pair forces, the
+// fixed-point j side of the tile passes, added in this order) scaled once.
+// One thread per component, so the stores are contiguous.  Explicit
+// roundings: the scales of the fixed-point terms are powers of two, so the
+// only rounded steps are the two additions and the last product, the ones
+// the host would do.  72 bytes read and 24 written per atom; the host did
+// this from nine pageable copies (100 us a call at 133 atoms, 437 at 20,566,
+// 20.6 ms at 568,384; with the one block 20 us, 59 us and 1.7 ms, most of it
+// the copy into the caller's pageable buffer).
+__global__ void k_forces_out(PackView v, double scale, double *out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 3 * v.n_atoms) return;
+  const int i = t / 3, k = t - 3 * i;
+  const long long *f = k == 0 ? v.fx : (k == 1 ? v.fy : v.fz);
+  const double *g = k == 0 ? v.gx : (k == 1 ? v.gy : v.gz);
+  const long long *h = k == 0 ? v.hx : (k == 1 ? v.hy : v.hz);
+  const double s = __dadd_rn(__dadd_rn(__dmul_rn((double)f[i], kInvForceScale), g[i]),
+                             __dmul_rn((double)h[i], kInvJScale));
+  out[t] = __dmul_rn(s, scale);
+}
+void launch_forces_out(const PackView &v, double scale, double *out, cudaStream_t st) {
+  if (v.n_atoms) PDGPU_LAUNCH(k_forces_out, (3 * v.n_atoms + 255) / 256, 256, 0, st, v, scale, out);
+}
+
 // The MD state in and out of pdgpu_md_run_io in one launch each: positions
 // (with the pair-kernel records) and velocities from / to interleaved
 // [n][3] staging blocks (either may be absent).

@@ -1,0 +1,29 @@
+"""Forces as the caller gets them: the device forms [n][3] in N from the
+accumulators.  Sizes on both sides of a block of the kernel (3 n components,
+256 a block), against the oracle's FP64 forces at the same coordinates
+(relative RMS 1e-5, the pair arithmetic's bound)."""
+import numpy as np
+import pytest
+
+from conftest import build_workspace, rel_rms
+from test_gpu_edge import _system
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [2, 85, 86, 171, 342])
+def test_forces_out_at_block_edges(n, gpu_ctx):
+    g = int(np.ceil(n ** (1.0 / 3.0)))
+    grid = np.array([[i, j, k] for i in range(g) for j in range(g) for k in range(g)], dtype=np.float64)[:n]
+    pos = 4.2 * grid + np.random.default_rng(n).normal(0.0, 0.2, (n, 3))
+    arrays, meta = _system(pos, np.arange(n) % 300)
+    ws, ff = build_workspace(arrays, meta, gpu_ctx)
+    ws.setPairPath(1)
+    ws.nlist().calcNewList()
+    ff.calcForces()
+    S = O.System(arrays, cutoff=float(meta["cutoff"]), inner=float(meta["inner"]))
+    f_ref, _, _ = S.calc_forces(pos, *S.nlist(pos))
+    assert rel_rms(ws.cur.f, f_ref) <= 1e-5
+    ws.close()
