@@ -207,7 +207,7 @@ struct PackView {
   int n_jc;                   // j-clusters over all systems
   const int *jc_atom0;        // [n_jc] first atom of each j-cluster
   const int *jc_off;          // [S+1] first j-cluster of each system
-  double *cbox;               // [6*n_jc] j-cluster boxes at the last search: lo xyz, hi xyz
+  float4 *cbox;               // [2*n_jc] j-cluster boxes at the last search, rounded outward: lo, hi
   double *xs;                 // [3*N] positions at the last tile search (x block, y block, z block)
   int4 *tile_meta;           // [tile_cap] per tile: first j atom, bond-order rows index (-1 none),
                               // i-cluster's first atom, system << 8 | (i atoms - 1) << 3 | (j atoms - 1)

@@ -183,240 +183,316 @@ __global__ void __launch_bounds__(128) k_tile_build(PackView v) {
 // same band and off-diagonal tables, so the tiles hold exactly the pairs a
 // list build at these positions would give them.
 //
-// (1) k_cluster_boxes: one thread per j-cluster folds its <= 8 atoms into
-// an FP64 box (a cluster with a NaN coordinate gets an infinite box: its
-// pairs are decided by the distance test alone) and saves the positions of
-// this rebuild (for a later list build at the same positions).
-// (2) k_tile_search: one block per i-cluster; its warps take the system's
-// j-clusters at or after the i-cluster 32 at a time, one per lane, and keep
-// those whose box lies within the list cutoff of the i-cluster's box (a
-// margin of 1e-9 relative keeps the cull conservative); for each kept
-// j-cluster the warp tests its 32 x 8 atom pairs (lane = i atom) and emits
-// a tile when any pair is in.
-__global__ void k_cluster_boxes(PackView v) {
-  const int jc = blockIdx.x * blockDim.x + threadIdx.x;
-  if (jc >= v.n_jc) return;
-  const int a0 = v.jc_atom0[jc];
-  const int s = v.sys_of[a0];
-  const int n = min(8, v.atom_off[s + 1] - a0);
+// (1) k_cluster_boxes: eight lanes per j-cluster fold its atoms into an FP32
+// box rounded outward (a cluster with a NaN coordinate gets an infinite box:
+// its pairs are decided by the distance test alone), save the positions of
+// this rebuild (for a later list build at the same positions) and clear the
+// tile counters.
+// (2) k_tile_search: one block per i-cluster.  Its threads take the system's
+// j-clusters at or after the i-cluster, one each, and put those whose box
+// may lie within the list cutoff of the i-cluster's box on a list in shared
+// memory (gaps rounded down, so the cull drops no pair); its warps then take
+// the list's entries in turn, test the 32 x 8 atom pairs (lane = i atom)
+// with the positions of the next entry already loading, and stage a tile
+// when any pair is in.
+//
+// What bounds it: latency (the pair tests of a 20,566-atom search are 3 us of
+// FP64 issue).  Chain neighbours sit next to one another, so of the groups
+// of 32 j-clusters that warps used to take whole, the first held nearly all
+// the candidates and one warp walked them one pair of loads at a time; with
+// the shared list the four warps get equal shares.  The FP32 boxes replace a
+// per-atom FP64 cull: they pass 11,140 candidates for 9,479 tiles on the
+// 16 x 80-residue system, 368 for 346 on a 64-residue peptide.
+// Measured (launch, ncu): 985 atoms 45 -> 8 us, 20,566 atoms 62 -> 15 us,
+// 64 OPLS peptides 150 -> 33 us, 512 peptides 671 -> 150 us.
+__global__ void __launch_bounds__(128) k_cluster_boxes(PackView v) {
+  PDGPU_DEP_ENTRY();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < 2) v.tile_count[t] = 0;
+  const int jc = t >> 3, k = t & 7;
+  const int q = min(jc, v.n_jc - 1);  // whole warps take part in the shuffles
+  const int a0 = v.jc_atom0[q];
+  const int n = min(8, v.atom_off[v.sys_of[a0] + 1] - a0);
   const int N = v.n_atoms;
-  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+  const int i = a0 + (k < n ? k : 0);
+  const double p[3] = {v.x[i], v.y[i], v.z[i]};
+  float lo[3], hi[3];
   bool wild = false;
-  for (int k = 0; k < n; k++) {
-    const int i = a0 + k;
-    const double p[3] = {v.x[i], v.y[i], v.z[i]};
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    wild |= !(p[c] == p[c]);
+    lo[c] = __double2float_rd(p[c]);
+    hi[c] = __double2float_ru(p[c]);
+    if (jc < v.n_jc && k < n) v.xs[(size_t)c * N + i] = p[c];
+  }
+  const unsigned g = 0xffu << (threadIdx.x & 24);  // this cluster's lanes
+  wild = (__ballot_sync(0xffffffffu, wild) & g) != 0;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
     for (int c = 0; c < 3; c++) {
-      wild |= !(p[c] == p[c]);
-      lo[c] = fmin(lo[c], p[c]);
-      hi[c] = fmax(hi[c], p[c]);
-      v.xs[(size_t)c * N + i] = p[c];
+      lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
+      hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
+    }
+  if (jc >= v.n_jc || k > 1) return;
+  const float w = k ? INFINITY : -INFINITY;
+  const float b[3] = {k ? hi[0] : lo[0], k ? hi[1] : lo[1], k ? hi[2] : lo[2]};
+  v.cbox[2 * (size_t)jc + k] = wild ? make_float4(w, w, w, 0.f) : make_float4(b[0], b[1], b[2], 0.f);
+}
+
+constexpr int kSearchWarps = 4;      // warps per i-cluster block of the tile search
+constexpr int kSearchThreads = 32 * kSearchWarps;
+// candidates held in shared memory: the cull takes that many j-clusters
+// between two rounds of pair tests, so the list cannot run over and the cull
+// has no barrier inside
+constexpr int kSearchCand = 1024;
+
+// Lower bound of the squared distance of two boxes (NaN gaps, from infinite
+// boxes, count as 0).
+__device__ __forceinline__ float box_gap2(const float4 &alo, const float4 &ahi, const float4 &blo,
+                                          const float4 &bhi) {
+  const float x = fmaxf(0.f, fmaxf(__fsub_rd(blo.x, ahi.x), __fsub_rd(alo.x, bhi.x)));
+  const float y = fmaxf(0.f, fmaxf(__fsub_rd(blo.y, ahi.y), __fsub_rd(alo.y, bhi.y)));
+  const float z = fmaxf(0.f, fmaxf(__fsub_rd(blo.z, ahi.z), __fsub_rd(alo.z, bhi.z)));
+  return __fadd_rd(__fadd_rd(__fmul_rd(x, x), __fmul_rd(y, y)), __fmul_rd(z, z));
+}
+
+// The bond-order bits (<= 2, == 3) of one candidate's pairs in `row` (some
+// lane's row is not empty, so the system has a band).  The eight band entries
+// load together, whether in the row or not: with a load under each bit's
+// branch a near-diagonal tile waited for eight of them in turn.
+__device__ __forceinline__ void search_orders(const PackView &v, unsigned row, int i, int li, int jb0, int o, int mid,
+                                              const signed char *band, bool has_off, unsigned &xr, unsigned &br) {
+  int bo[8];
+  unsigned inb = 0;
+#pragma unroll
+  for (int t = 0; t < 8; t++) {
+    const int delta = jb0 + t - o - li;  // j > i wherever the row has a bit
+    const bool in = ((row >> t) & 1u) && delta < mid;
+    inb |= (unsigned)in << t;
+    bo[t] = band[in ? (long long)li * mid + (delta - 1) : 0];
+  }
+#pragma unroll
+  for (int t = 0; t < 8; t++) {
+    if (((inb >> t) & 1u) && bo[t] <= 2) xr |= 1u << t;
+    if (((inb >> t) & 1u) && bo[t] == 3) br |= 1u << t;
+  }
+  if (has_off) {
+    const unsigned rest = row & ~inb;  // beyond the band: the off-diagonal partners
+    for (int k = v.off_ptr[i], e = v.off_ptr[i + 1]; k < e; k++) {
+      const int2 q = v.off_data[k];
+      const int t = q.x - jb0;
+      if (t < 0 || t > 7 || !((rest >> t) & 1u)) continue;
+      if ((q.y & 7) <= 2) xr |= 1u << t;
+      if ((q.y & 7) == 3) br |= 1u << t;
     }
   }
-  for (int c = 0; c < 3; c++) {
-    v.cbox[6 * (size_t)jc + c] = wild ? -INFINITY : lo[c];
-    v.cbox[6 * (size_t)jc + 3 + c] = wild ? INFINITY : hi[c];
-  }
 }
-
-constexpr int kSearchWarps = 8;  // warps per i-cluster block of the tile search
-
-// One candidate j-cluster against this lane's i atom: the pair bits and
-// the bond-order bits (<= 2, == 3).  The pair tests come first (the 8 j
-// positions load independently), then the bond orders of the pairs in
-// (independent band loads).
-struct SearchRow {
-  unsigned row, xr, br;
-};
-__device__ __forceinline__ SearchRow search_row(const PackView &v, bool live, int i, int li, int a0, double xi,
-                                                double yi, double zi, double lim, int jb0, int nb, int o,
-                                                int mid, const signed char *band, bool has_off, int s) {
-  SearchRow r = {0u, 0u, 0u};
-  if (!live) return r;
-#pragma unroll
-  for (int t = 0; t < 8; t++) {
-    const int j = jb0 + t;
-    // the half list: j > i inside the i-cluster
-    if (t < nb && !(j <= i && j < a0 + 32) && !(ref_d2(xi, yi, zi, v.x[j], v.y[j], v.z[j]) > lim))
-      r.row |= 1u << t;
-  }
-#pragma unroll
-  for (int t = 0; t < 8; t++) {
-    if (!((r.row >> t) & 1u)) continue;
-    const int lj = jb0 + t - o;
-    const int delta = lj > li ? lj - li : li - lj;
-    int bo = 7;
-    if (delta < mid)
-      bo = band[(long long)min(li, lj) * mid + (delta - 1)];
-    else if (has_off)
-      bo = bond_order(v, s, i, jb0 + t);
-    if (bo <= 2)
-      r.xr |= 1u << t;
-    else if (bo == 3)
-      r.br |= 1u << t;
-  }
-  return r;
-}
-// A search block's tiles are staged in shared memory and written to the
-// tile store as one contiguous range by the block's last warp to finish, so
-// the tiles of an i-cluster sit together and a pass that walks contiguous
-// tile ranges meets few i-cluster changes (each one a reload of the i side).
-// Tiles beyond the staging capacity go to the store one at a time.
-constexpr int kSearchStage = 256;
+// A search block's tiles (and their bond-order rows) are staged in shared
+// memory and written to the tile store as one contiguous range, so the tiles
+// of an i-cluster sit together and a pass that walks contiguous tile ranges
+// meets few i-cluster changes (each one a reload of the i side), and one
+// atomic per block and counter reserves the space.  What does not fit the
+// stage goes to the store one at a time.
+constexpr int kSearchStage = 256, kSearchSpec = 24;
 struct SearchStage {
-  int n;                               // tiles emitted into the stage (may pass kSearchStage)
-  int done;                            // warps that have finished their j-clusters
-  int4 meta[kSearchStage];
+  int n, nspec;                        // emitted (may pass the capacities)
+  int base, sbase;                     // first slots in the store
+  int4 meta[kSearchStage];             // y: -1, the staged rows' index, or -2 - the store's index
   unsigned rows[kSearchStage * 8];     // byte l of tile k's 32 bytes = i lane l's bits
+  unsigned spec[kSearchSpec * 16];
 };
-// Store one tile (when any pair is in); false when a capacity ran out
-// (cannot happen: the capacities are worst cases).
-__device__ __forceinline__ bool search_emit(const PackView &v, int lane, const SearchRow &r, int jb0, int a0, int s,
-                                            int na, int nb, SearchStage &stage) {
-  if (!__any_sync(0xffffffffu, r.row != 0)) return true;
-  int spec = -1;
-  if (__any_sync(0xffffffffu, (r.xr | r.br) != 0)) {
-    if (lane == 0) spec = atomicAdd(&v.tile_count[1], 1);
-    spec = __shfl_sync(0xffffffffu, spec, 0);
-    if (spec >= v.spec_cap) {
+// Store one tile that holds a pair; false when a capacity ran out (cannot
+// happen: the capacities are worst cases).
+__device__ __forceinline__ bool search_emit(const PackView &v, int lane, unsigned row, unsigned xr, unsigned br,
+                                            int jb0, int a0, int s, int na, int nb, SearchStage &stage) {
+  const bool special = __any_sync(0xffffffffu, (xr | br) != 0);
+  int k = 0, spec = -1;
+  if (lane == 0) {
+    k = atomicAdd(&stage.n, 1);
+    if (special && k < kSearchStage) spec = atomicAdd(&stage.nspec, 1);
+  }
+  k = __shfl_sync(0xffffffffu, k, 0);
+  spec = __shfl_sync(0xffffffffu, spec, 0);
+  const bool staged = k < kSearchStage;
+  int e = k;  // a tile past the stage: its slot in the store
+  if (!staged) {
+    if (lane == 0) e = atomicAdd(&v.tile_count[0], 1);
+    e = __shfl_sync(0xffffffffu, e, 0);
+    if (e >= v.tile_cap) {
       if (lane == 0) atomicExch(&v.flags[F_NL_OVERFLOW], 1);
       return false;
     }
-    reinterpret_cast<unsigned char *>(v.spec_rows)[64 * (size_t)spec + lane] = (unsigned char)r.xr;
-    reinterpret_cast<unsigned char *>(v.spec_rows)[64 * (size_t)spec + 32 + lane] = (unsigned char)r.br;
   }
-  const int4 meta = make_int4(jb0, spec, a0, (s << 8) | ((na - 1) << 3) | (nb - 1));
-  int k = 0;
-  if (lane == 0) k = atomicAdd(&stage.n, 1);
-  k = __shfl_sync(0xffffffffu, k, 0);
-  if (k < kSearchStage) {
-    reinterpret_cast<unsigned char *>(stage.rows)[32 * k + lane] = (unsigned char)r.row;
-    if (lane == 0) stage.meta[k] = meta;
-    return true;
+  if (special) {
+    unsigned char *to = reinterpret_cast<unsigned char *>(stage.spec) + 64 * spec;
+    if (!staged || spec >= kSearchSpec) {
+      int se = 0;
+      if (lane == 0) se = atomicAdd(&v.tile_count[1], 1);
+      se = __shfl_sync(0xffffffffu, se, 0);
+      if (se >= v.spec_cap) {
+        if (lane == 0) atomicExch(&v.flags[F_NL_OVERFLOW], 1);
+        return false;
+      }
+      spec = staged ? -2 - se : se;
+      to = reinterpret_cast<unsigned char *>(v.spec_rows) + 64 * (size_t)se;
+    }
+    to[lane] = (unsigned char)xr;
+    to[32 + lane] = (unsigned char)br;
   }
-  int e = 0;
-  if (lane == 0) e = atomicAdd(&v.tile_count[0], 1);
-  e = __shfl_sync(0xffffffffu, e, 0);
-  if (e >= v.tile_cap) {
-    if (lane == 0) atomicExch(&v.flags[F_NL_OVERFLOW], 1);
-    return false;
-  }
-  reinterpret_cast<unsigned char *>(v.tile_rows)[32 * (size_t)e + lane] = (unsigned char)r.row;
-  if (lane == 0) v.tile_meta[e] = meta;
+  unsigned char *rows = staged ? reinterpret_cast<unsigned char *>(stage.rows)
+                               : reinterpret_cast<unsigned char *>(v.tile_rows);
+  rows[32 * (size_t)e + lane] = (unsigned char)row;
+  if (lane == 0) (staged ? stage.meta : v.tile_meta)[e] = make_int4(jb0, spec, a0, (s << 8) | ((na - 1) << 3) | (nb - 1));
   return true;
 }
 
-__global__ void __launch_bounds__(32 * kSearchWarps, 5) k_tile_search(PackView v) {
+__global__ void __launch_bounds__(kSearchThreads) k_tile_search(PackView v) {
+  // everything but the boxes and the counters is older than k_cluster_boxes:
+  // it is read while that kernel still runs
   const int sc = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int s = v.sc_sys[sc];
   const int a0 = v.sc_atom0[sc];
   const int end = v.atom_off[s + 1];
   const int na = min(32, end - a0);
-  const int jc0 = v.sc_jc0[sc], jc_end = v.jc_off[s + 1];
+  const int jc0 = v.sc_jc0[sc], jcs = v.jc_off[s], jc_end = v.jc_off[s + 1];
   const double lim = v.sp[s].nl_lim2_d;
-  const double cull = lim * (1.0 + 1e-9);
-  // the i-cluster's box: its (up to four) j-clusters' boxes
-  double ilo[3] = {INFINITY, INFINITY, INFINITY}, ihi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  for (int q = 0; q < 4 && jc0 + q < jc_end; q++)
-    for (int c = 0; c < 3; c++) {
-      ilo[c] = fmin(ilo[c], v.cbox[6 * (size_t)(jc0 + q) + c]);
-      ihi[c] = fmax(ihi[c], v.cbox[6 * (size_t)(jc0 + q) + 3 + c]);
-    }
-  // this lane's i atom and what its bond orders need
+  const float cull = __double2float_ru(lim);
   const bool live = lane < na;
   const int i = a0 + (live ? lane : 0);
   const double xi = v.x[i], yi = v.y[i], zi = v.z[i];
   const int o = v.atom_off[s], mid = v.mid[s], li = i - o;
   const signed char *band = reinterpret_cast<const signed char *>(v.band) + v.band_off[s];
   const bool has_off = v.off_ptr[i + 1] > v.off_ptr[i];
-  // the i atoms' positions for the per-atom cull
-  __shared__ double sx[32], sy[32], sz[32];
+  const bool any_off = __any_sync(0xffffffffu, has_off);
   __shared__ SearchStage stage;
-  __shared__ int stop_s;  // an earlier overflow, read once so every thread of the block agrees
-  if (threadIdx.x == 0) {
-    stage.n = 0;
-    stage.done = 0;
-    stop_s = v.flags[F_NL_OVERFLOW];
-  }
+  __shared__ int cand[kSearchCand];
+  __shared__ int ncand, stop_s;  // stop_s: an earlier overflow, read once so every thread agrees
+  __shared__ double sj[kSearchWarps][3][8];
+  __shared__ float4 ilo_s[32], ihi_s[32];  // the i atoms, rounded down and up
   if (warp == 0) {
-    sx[lane] = xi;
-    sy[lane] = yi;
-    sz[lane] = zi;
+    ilo_s[lane] = make_float4(__double2float_rd(xi), __double2float_rd(yi), __double2float_rd(zi), 0.f);
+    ihi_s[lane] = make_float4(__double2float_ru(xi), __double2float_ru(yi), __double2float_ru(zi), 0.f);
   }
+  if (threadIdx.x == 0) {
+    stage.n = stage.nspec = 0;
+    ncand = 0;
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (threadIdx.x == 0) stop_s = v.flags[F_NL_OVERFLOW];
+  // the i-cluster's box: its (up to four) j-clusters' boxes
+  float4 ilo = v.cbox[2 * (size_t)jc0], ihi = v.cbox[2 * (size_t)jc0 + 1];
+  for (int q = 1; q < 4 && jc0 + q < jc_end; q++) {
+    const float4 l = v.cbox[2 * (size_t)(jc0 + q)], h = v.cbox[2 * (size_t)(jc0 + q) + 1];
+    ilo = make_float4(fminf(ilo.x, l.x), fminf(ilo.y, l.y), fminf(ilo.z, l.z), 0.f);
+    ihi = make_float4(fmaxf(ihi.x, h.x), fmaxf(ihi.y, h.y), fmaxf(ihi.z, h.z), 0.f);
+  }
+  // An i-cluster across the end of one chain and the start of the next has a
+  // box as long as the chains (647 j-clusters passed it on the 16 x 80-residue
+  // system, and that block took 88 us).  Where the box is wider than the
+  // cutoff, one of the i-cluster's j-cluster boxes must also lie within the
+  // cutoff of the candidate's, and for one of those that is as wide, one of
+  // its atoms.  Ordinary clusters (10-12 A) pass about as many either way.
+  const float reach = sqrtf(cull);
+  const bool wide = !(ihi.x - ilo.x <= reach && ihi.y - ilo.y <= reach && ihi.z - ilo.z <= reach);
   __syncthreads();
   if (stop_s) return;
   bool ok = true;  // false once a capacity ran out (warp-uniform)
-  for (int base = jc0 + 32 * warp; ok && base < jc_end; base += 32 * kSearchWarps) {
-    bool cand = false;
-    const int jc = base + lane;
-    if (jc < jc_end) {
-      double jlo[3], jhi[3];
-      for (int c = 0; c < 3; c++) {
-        jlo[c] = v.cbox[6 * (size_t)jc + c];
-        jhi[c] = v.cbox[6 * (size_t)jc + 3 + c];
-      }
-      double g2 = 0.0;
-      for (int c = 0; c < 3; c++) {
-        const double gap = fmax(0.0, fmax(jlo[c] - ihi[c], ilo[c] - jhi[c]));
-        g2 += gap * gap;
-      }
-      cand = !(g2 > cull);  // NaN (infinite boxes): a candidate
-      // boxes this close: some i atom must lie within the cutoff of the
-      // j-cluster's box (an i-cluster across two chains has a large box)
-      if (cand) {
-        cand = false;
-        for (int k = 0; k < na && !cand; k++) {
-          const double p[3] = {sx[k], sy[k], sz[k]};
-          double h2 = 0.0;
-          for (int c = 0; c < 3; c++) {
-            const double gap = fmax(0.0, fmax(jlo[c] - p[c], p[c] - jhi[c]));
-            h2 += gap * gap;
+  const int axis = min(lane >> 3, 2);  // lanes 0-23 load a candidate's x, y, z
+  const double *src = axis == 0 ? v.x : (axis == 1 ? v.y : v.z);
+  for (int base = jc0; base < jc_end; base += kSearchCand) {
+    // cull: one j-cluster per thread and turn, the next turn's boxes loading
+    const int stop = min(base + kSearchCand, jc_end);
+    const int first = base + (int)threadIdx.x;
+    float4 nlo = v.cbox[2 * (size_t)min(first, jc_end - 1)], nhi = v.cbox[2 * (size_t)min(first, jc_end - 1) + 1];
+    for (int j0 = base + 32 * warp; j0 < stop; j0 += kSearchThreads) {
+      const int jc = j0 + lane, jn = min(jc + kSearchThreads, jc_end - 1);
+      const float4 jlo = nlo, jhi = nhi;
+      nlo = v.cbox[2 * (size_t)jn];
+      nhi = v.cbox[2 * (size_t)jn + 1];
+      bool in = jc < stop && !(box_gap2(ilo, ihi, jlo, jhi) > cull);
+      if (wide && in) {
+        in = false;
+        for (int q = 0; q < 4 && jc0 + q < jc_end; q++) {
+          const float4 l = v.cbox[2 * (size_t)(jc0 + q)], h = v.cbox[2 * (size_t)(jc0 + q) + 1];
+          bool near = !(box_gap2(l, h, jlo, jhi) > cull);
+          if (near && !(h.x - l.x <= reach && h.y - l.y <= reach && h.z - l.z <= reach)) {
+            near = false;
+#pragma unroll
+            for (int k = 0; k < 8; k++) near |= !(box_gap2(ilo_s[8 * q + k], ihi_s[8 * q + k], jlo, jhi) > cull);
           }
-          cand = !(h2 > cull);
+          in |= near;
         }
       }
+      const unsigned m = __ballot_sync(0xffffffffu, in);
+      if (m) {
+        int at = 0;
+        if (lane == 0) at = atomicAdd(&ncand, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (in) cand[at + __popc(m & ((1u << lane) - 1u))] = jc;
+      }
     }
-    unsigned m = __ballot_sync(0xffffffffu, cand);
-    // two candidates at a time: their loads overlap
-    while (ok && m) {
-      const int q1 = __ffs(m) - 1;
-      m &= m - 1;
-      const int q2 = m ? __ffs(m) - 1 : -1;
-      if (m) m &= m - 1;
-      const int jb1 = v.jc_atom0[base + q1], nb1 = min(8, end - jb1);
-      const int jb2 = q2 >= 0 ? v.jc_atom0[base + q2] : jb1, nb2 = min(8, end - jb2);
-      const SearchRow r1 = search_row(v, live, i, li, a0, xi, yi, zi, lim, jb1, nb1, o, mid, band, has_off, s);
-      SearchRow r2 = {0u, 0u, 0u};
-      if (q2 >= 0) r2 = search_row(v, live, i, li, a0, xi, yi, zi, lim, jb2, nb2, o, mid, band, has_off, s);
-      ok = search_emit(v, lane, r1, jb1, a0, s, na, nb1, stage);
-      if (ok && q2 >= 0) ok = search_emit(v, lane, r2, jb2, a0, s, na, nb2, stage);
+    __syncthreads();
+    const int n = ncand;
+    // the pair tests: a candidate per warp, the next two's positions loading
+    // (a j-cluster's first atom follows from its index: no load before them)
+    auto fetch = [&](int c, int &jb0) {
+      jb0 = o + 8 * (cand[min(c, n - 1)] - jcs);
+      return src[min(jb0 + (lane & 7), end - 1)];
+    };
+    int jb1 = 0, jb2 = 0;
+    double p1 = 0.0, p2 = 0.0;
+    if (warp < n) {
+      p1 = fetch(warp, jb1);
+      p2 = fetch(warp + kSearchWarps, jb2);
     }
+    for (int c = warp; ok && c < n; c += kSearchWarps) {
+      __syncwarp();
+      if (lane < 24) sj[warp][axis][lane & 7] = p1;
+      __syncwarp();
+      const int jb = jb1, nj = min(8, end - jb);
+      p1 = p2;
+      jb1 = jb2;
+      p2 = fetch(c + 2 * kSearchWarps, jb2);
+      unsigned row = 0;
+#pragma unroll
+      for (int t = 0; t < 8; t++)
+        if (!(ref_d2(xi, yi, zi, sj[warp][0][t], sj[warp][1][t], sj[warp][2][t]) > lim)) row |= 1u << t;
+      row &= (1u << nj) - 1u;
+      // the half list: j > i inside the i-cluster
+      if (jb < a0 + 32 && i >= jb) row &= i - jb >= 7 ? 0u : ~((2u << (i - jb)) - 1u);
+      if (!live) row = 0;
+      if (__any_sync(0xffffffffu, row != 0)) {
+        unsigned xr = 0, br = 0;
+        if (any_off || jb - (a0 + na - 1) < mid) search_orders(v, row, i, li, jb, o, mid, band, has_off, xr, br);
+        ok = search_emit(v, lane, row, xr, br, jb, a0, s, na, nj, stage);
+      }
+    }
+    __syncthreads();  // the list has been read
+    if (threadIdx.x == 0) ncand = 0;
+    if (stop < jc_end) __syncthreads();
   }
-  // the staged tiles as one range of the tile store, written by the last
-  // warp to finish; the others exit at once (a warp with no j-clusters does
-  // not hold its slot while the block's busy warps run)
-  __syncwarp();
-  __threadfence_block();  // this warp's stage writes before its count
-  int last = 0;
-  if (lane == 0) last = atomicAdd(&stage.done, 1) == kSearchWarps - 1;
-  last = __shfl_sync(0xffffffffu, last, 0);
-  if (!last) return;
-  __syncwarp();
-  __threadfence_block();  // every warp's stage writes after the count
-  const int n = min(*(volatile int *)&stage.n, kSearchStage);
+  const int n = min(stage.n, kSearchStage), ns = min(stage.nspec, kSearchSpec);
   if (n == 0) return;
-  long long b0 = 0;
-  if (lane == 0) b0 = atomicAdd(&v.tile_count[0], n);
-  b0 = __shfl_sync(0xffffffffu, b0, 0);
-  if (b0 + n > v.tile_cap) {
-    if (lane == 0) atomicExch(&v.flags[F_NL_OVERFLOW], 1);
+  if (threadIdx.x == 0) stage.base = atomicAdd(&v.tile_count[0], n);
+  if (threadIdx.x == 32) stage.sbase = ns ? atomicAdd(&v.tile_count[1], ns) : 0;
+  __syncthreads();
+  const long long b0 = stage.base, s0 = stage.sbase;
+  if (b0 + n > v.tile_cap || s0 + ns > v.spec_cap) {
+    if (threadIdx.x == 0) atomicExch(&v.flags[F_NL_OVERFLOW], 1);
     return;
   }
-  const volatile unsigned *rows = stage.rows;
-  for (int w = lane; w < 8 * n; w += 32) v.tile_rows[8 * b0 + w] = rows[w];
-  for (int k = lane; k < n; k += 32) {
-    const volatile int *m = reinterpret_cast<const volatile int *>(&stage.meta[k]);
-    v.tile_meta[b0 + k] = make_int4(m[0], m[1], m[2], m[3]);
+  for (int w = threadIdx.x; w < 8 * n; w += kSearchThreads) v.tile_rows[8 * b0 + w] = stage.rows[w];
+  for (int w = threadIdx.x; w < 16 * ns; w += kSearchThreads) v.spec_rows[16 * s0 + w] = stage.spec[w];
+  for (int k = threadIdx.x; k < n; k += kSearchThreads) {
+    int4 m = stage.meta[k];
+    if (m.y >= 0)
+      m.y += (int)s0;
+    else if (m.y < -1)
+      m.y = -2 - m.y;
+    v.tile_meta[b0 + k] = m;
   }
 }
 
@@ -834,9 +910,8 @@ void launch_tiles_build(const PackView &v, cudaStream_t st) {
 }
 void launch_tiles_search(const PackView &v, cudaStream_t st) {
   if (!v.n_sc) return;
-  cudaMemsetAsync(v.tile_count, 0, 2 * sizeof(int), st);
-  PDGPU_LAUNCH(k_cluster_boxes, (v.n_jc + 127) / 128, 128, 0, st, v);
-  PDGPU_LAUNCH(k_tile_search, v.n_sc, 32 * kSearchWarps, 0, st, v);
+  PDGPU_LAUNCH_DEP(k_cluster_boxes, (v.n_jc + 15) / 16, 128, 0, st, v);
+  PDGPU_LAUNCH_DEP(k_tile_search, v.n_sc, kSearchThreads, 0, st, v);
 }
 void launch_born_radii_tile(const PackView &v, cudaStream_t st, int zero_first) {
   if (!v.n_sc) return;
