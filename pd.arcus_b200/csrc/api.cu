@@ -1318,12 +1318,9 @@ void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepS
   const bool surf = P.v.lc.update > 0;
   const bool side = bonded || surf;
   if (side) {
-    const size_t bytes = sizeof(long long) * (size_t)P.v.n_atoms;
     cudaEventRecord(P.fork, st);
     cudaStreamWaitEvent(P.side, P.fork, 0);
-    cudaMemsetAsync(P.v.fx, 0, bytes, P.side);
-    cudaMemsetAsync(P.v.fy, 0, bytes, P.side);
-    cudaMemsetAsync(P.v.fz, 0, bytes, P.side);
+    cudaMemsetAsync(P.v.fx, 0, sizeof(long long) * 3 * (size_t)P.v.n_atoms, P.side);  // fx, fy, fz: one block
     if (bonded) launch_bonded_terms(P.v, P.side);
     if (surf) launch_lcpo(P.v, P.side, step, false, P.csr_stale);
     cudaEventRecord(P.join, P.side);

@@ -509,9 +509,9 @@ Pack *pack_create(int device, cudaStream_t st, const std::vector<const SystemHos
   PALLOC(v.gx, N);
   PALLOC(v.gy, N);
   PALLOC(v.gz, N);
-  PALLOC(v.fx, N);
-  PALLOC(v.fy, N);
-  PALLOC(v.fz, N);
+  PALLOC(v.fx, 3 * (size_t)N);  // one block: zeroed by one memset
+  v.fy = v.fx + N;
+  v.fz = v.fx + 2 * (size_t)N;
   PALLOC(v.fox, N);
   PALLOC(v.foy, N);
   PALLOC(v.foz, N);
