@@ -531,8 +531,8 @@ int pdgpu_profile_pair_kernels(pdgpu_ctx *ctx, int32_t sys, int32_t reps, double
 /* Instrumentation (no reference counterpart): device times (CUDA events on
  * the context stream, averaged over reps) of the evaluation kernel on the
  * cluster-pair tiles: ms[0..2] its Born-sum, GB + LJ + Coulomb and
- * chain-rule phases as three launches, ms[3] the three in one cooperative
- * launch (the form the protocols run).  counts (NULL, or 5 entries):
+ * chain-rule phases as three launches (the form the protocols run), ms[3]
+ * the three in one cooperative launch.  counts (NULL, or 5 entries):
  * [0] tiles, [1] tiles the chain-rule phase visited (a pair inside the
  * Still cutoff), [2..4] tiles the Born-sum, GB + LJ + Coulomb and
  * chain-rule phases redid in their careful form (a pair at a decision
@@ -547,11 +547,9 @@ int pdgpu_profile_eval(pdgpu_ctx *ctx, int32_t sys, int32_t reps, double *ms, in
 int pdgpu_measure_pipe_peaks(pdgpu_ctx *ctx, double *out);
 /* How an evaluation on the tile layout is launched (no reference
  * counterpart): 1 = the three passes in one cooperative launch everywhere,
- * 0 = the same three phases as three launches everywhere, 2 (the default) =
- * one cooperative launch for single evaluations and minimiser / Monte Carlo
- * steps, three launches inside MD step blocks (where the next step's first
- * phase can start beside the bonded terms and the previous step's energy
- * record); -1 = only report.  Every mode gives the same bits.  *current
+ * 0 = as three launches everywhere, 2 (the default) = the faster form for
+ * each use (three dependent launches, at every size and in every loop
+ * measured); -1 = only report.  Every mode gives the same bits.  *current
  * (may be NULL) receives the mode. */
 int pdgpu_eval_mode(pdgpu_ctx *ctx, int32_t sys, int32_t set, int32_t *current);
 /* Device times (CUDA events, averaged over reps full evaluations at step 0)

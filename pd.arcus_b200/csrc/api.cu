@@ -76,7 +76,7 @@ static int barrier_check(pdgpu_ctx *c, pdgpu::Pack &P, const int *flags_host = n
   int f = 0;
   if (flags_host) {
     f = flags_host[F_BARRIER];
-  } else if (P.v.tile_mode) {
+  } else if (P.v.tile_mode && P.coop) {  // (the three launches have no barrier)
     PDGPU_CUDA(cudaMemcpyAsync(&f, P.v.flags + F_BARRIER, sizeof f, cudaMemcpyDeviceToHost, c->st));
     int r = sync_check(c, "evaluation flags");
     if (r) return r;
@@ -2226,16 +2226,16 @@ int pdgpu_eval_mode(pdgpu_ctx *c, int32_t sys, int32_t set, int32_t *current) {
   Pack &P = *e->pack;
   if (set < -1 || set > 2) {
     set_error("pdgpu_eval_mode: set must be -1 (query), 0 (three launches), 1 (one cooperative launch) or 2 "
-              "(cooperative for single evaluations, three launches inside MD step blocks)");
+              "(the faster form for each use)");
     return PDGPU_ERR_ARG;
   }
   if (set >= 0) {
-    const bool one = set >= 1, md = set == 1;
-    if (P.coop_md != md) e->drop_graph();
-    P.coop = one;
-    P.coop_md = md;
+    const bool one = set == 1;
+    if (P.coop_md != one) e->drop_graph();
+    P.eval_mode = set;
+    P.coop = P.coop_md = one;
   }
-  if (current) *current = P.coop ? (P.coop_md ? 1 : 2) : 0;
+  if (current) *current = P.coop ? (P.coop_md ? 1 : 2) : P.eval_mode;
   return PDGPU_OK;
 }
 

@@ -1,4 +1,4 @@
-// One GB evaluation on the cluster-pair tiles in one persistent launch.
+// One GB evaluation on the cluster-pair tiles.
 //
 // FF_GeneralizedBorn_Still::calcForces in FastMode (gbff.cpp:168-180) has
 // three passes over the pairs with a global dependency between each:
@@ -8,14 +8,28 @@
 //      needs every radius, and leaves each atom's dE/da complete only when
 //      every pair is in
 //   C  Born-radius chain rule (loop 2, :1751-1818); needs every dE/da.
-// Here the three are phases of one cooperative launch (every block
-// resident), separated by two grid barriers.  The per-atom steps between
+// They run as three launches of persistent grids, each a dependent launch
+// that loads its first tiles' older records before it waits for the phase
+// before, or as the phases of one cooperative launch (every block resident)
+// with two grid barriers (pdgpu_eval_mode 1).  The per-atom steps between
 // them are folded into the phases: phase B forms each atom's Born radius
 // from its fixed-point sum when it stages the atom (the FP64 expression of
 // k_born_finish, so the same bits), and phase C forms each atom's chain
 // weight gpi * dE/da the same way.  The per-atom outputs (Born radii, the
 // per-atom energies) are written by grid-stride epilogues that nothing in
 // the same phase reads.
+//
+// Every phase has its own build (the template's PH), because what bounds the
+// phases includes fetching their instructions: the one kernel that held all
+// three was 126 KB of code, a warp of a small system runs each part of it
+// once per launch, and a quarter of its stalls were on instruction fetch
+// (ncu, 985 atoms).  The builds are 32, 55 and 43 KB and get the registers
+// their phase needs (no spills in A and B).  Measured, one launch of all
+// three / three launches of it / three builds: MD at 20,566 atoms - / 65.4 /
+// 63.8 us a step, 64 OPLS peptides - / 219 / 212 us a step; a call of
+// pdgpu_calc_forces 52 / 49 / 46 us at 985 atoms, 92 / - / 82 at 20,566,
+// 907 / - / 888 for 512 peptides.  So every caller uses the three launches;
+// the cooperative form stays for callers that ask for it.
 //
 // Every warp keeps one contiguous tile range for phases A and B (an equal
 // share of the pack's tiles).  Phase A also notes the tiles that hold a
@@ -27,9 +41,7 @@
 //
 // The barriers spin with a bounded number of naps; a barrier that runs out
 // sets F_BARRIER, and every block then returns (the host reports it and
-// clears the counter).  The same kernel runs one phase per launch where a
-// cooperative launch is not available (PDGPU_FUSED=0, or a grid that cannot
-// be resident): three launches, the same arithmetic, the same results.
+// clears the counter).  PDGPU_FUSED=0 turns the cooperative form off.
 //
 // Pair arithmetic: the phase-A Born terms are those of the row and tile
 // passes (born_term_noV, explicit roundings: the same Born radii bit for
@@ -48,8 +60,11 @@
 namespace pdgpu {
 
 constexpr int kEvWarps = 4;  // warps per block
-// resident blocks per SM the register allocation must allow: 4 (up to 128
-// registers a thread; the default), or 5 (PDGPU_EV_BLOCKS=5; 102 registers)
+// resident blocks per SM the register allocation must allow (up to 128
+// registers a thread).  With five for phases A and C 64 OPLS peptides ran 1 %
+// faster a step and 985 atoms 1.4 % slower; with six or eight every size was
+// slower, phase B with five 6 % slower.
+constexpr int kEvBlocks = 4;
 constexpr unsigned kBarrierNaps = 1u << 22;  // about half a second of 100 ns naps
 
 // ------------------------------------------------------------- barrier
@@ -66,13 +81,16 @@ __device__ __forceinline__ void griddep_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 // Grid barrier over a counter that counts arrivals; every block waits for
-// `target` arrivals.  False when the wait ran out (the flag is set).
+// `target` arrivals.  False when the wait ran out (the flag is set).  The
+// arrival releases what the block wrote (ordered before it by the block
+// barrier) and returns nothing, and a poll that sees the target acquires what
+// the others wrote: the last block to arrive passes after one poll (2,700
+// cycles with fences around an atomic that returned its value, 2,000 now).
 __device__ __forceinline__ bool grid_barrier(unsigned *ctr, unsigned target, int *flags) {
   __shared__ int ok_s;
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(ctr, 1u);
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
     int ok = 1;
     unsigned naps = 0;
     while (ld_acquire_u32(ctr) < target) {
@@ -81,18 +99,25 @@ __device__ __forceinline__ bool grid_barrier(unsigned *ctr, unsigned target, int
         atomicExch(&flags[F_BARRIER], 1);
         break;
       }
-      __nanosleep(100);
+      if (naps > 64) __nanosleep(100);  // (a phase's tail is short: the first polls are back to back)
     }
-    __threadfence();
     ok_s = ok;
   }
   __syncthreads();
   return ok_s != 0;
 }
 
-// This warp's share [e0, e1) of T work items.
-__device__ __forceinline__ void ev_range(long long T, int warp, int &e0, int &e1) {
-  const long long G = (long long)gridDim.x * kEvWarps;
+// Blocks of the launch that take part: one warp per tile at most, enough
+// threads for one atom each.  The grid is sized for the pack's worst case
+// (1,984 warps at 985 atoms, which has 347 tiles); the blocks past the active
+// ones leave at once, so the barriers and the exit count fewer arrivals.
+__device__ __forceinline__ int ev_active(const PackView &v) {
+  const int need = max((v.tile_count[0] + kEvWarps - 1) / kEvWarps, (v.n_atoms + 32 * kEvWarps - 1) / (32 * kEvWarps));
+  return min((int)gridDim.x, max(need, 1));
+}
+// This warp's share [e0, e1) of T work items, over `blocks` blocks.
+__device__ __forceinline__ void ev_range(long long T, int blocks, int warp, int &e0, int &e1) {
+  const long long G = (long long)blocks * kEvWarps;
   const long long g = (long long)blockIdx.x * kEvWarps + warp;
   e0 = (int)(T * g / G);
   e1 = (int)(T * (g + 1) / G);
@@ -311,7 +336,7 @@ __device__ __forceinline__ BornTileOut born_tile(const ExactIn &v, const BornTil
     // the j side's term is made fixed point by the lane that owns j (the same bits)
     const float tJ = ok ? __fmul_rn(term, q.Vi) : 0.f;
     tile_i += __float2ll_rn(ok ? __fmul_rn(term, jc.y) : 0.f);
-    jacc += __float2ll_rn(__shfl_sync(0xffffffffu, tJ, g8 | ((a - t) & 7)));
+    jacc += __float2ll_rn(t == 0 ? tJ : __shfl_sync(0xffffffffu, tJ, g8 | ((a - t) & 7)));
   }
   BornTileOut o;
   o.tile_i = tile_i;
@@ -351,10 +376,10 @@ __device__ __forceinline__ void born_add_j(const PackView &v, const TileInfo &ti
   if (lane < ti.nb && jacc) atomicAdd((unsigned long long *)&v.bsum[ti.b0 + lane], (unsigned long long)jacc);
 }
 
-__device__ __forceinline__ void phase_born(const PackView &v, int warp, int lane, float4 (*sA)[16],
+__device__ __forceinline__ void phase_born(const PackView &v, int blocks, int warp, int lane, float4 (*sA)[16],
                                            float4 (*sB)[16], float4 (*sC)[16]) {
   int e, e1;
-  ev_range(v.tile_count[0], warp, e, e1);
+  ev_range(v.tile_count[0], blocks, warp, e, e1);
   const int first = e;
   const int g8 = lane & ~7, a = lane & 7;
   int a0 = -1, na = 0, nd = 0;
@@ -381,6 +406,7 @@ __device__ __forceinline__ void phase_born(const PackView &v, int warp, int lane
     near = 0;
     run0 = upto;
   };
+#pragma unroll 1
   for (; e < e1; e++) {
     int te;
     const EvStage cur = walk.next(v, lane, te);
@@ -415,6 +441,7 @@ __device__ __forceinline__ void phase_born(const PackView &v, int warp, int lane
   if (v.defer_stats && lane == 0 && nd) atomicAdd(&v.defer_stats[0], nd);
   // the deferred tiles in the careful form
   __syncwarp();
+#pragma unroll 1
   for (int k = 0; k < nd; k++) {
     const int t = v.defer_list[first + k];
     const EvStage cur = ev_stage_one<1>(v, t, lane);
@@ -546,7 +573,7 @@ struct ISide {
     bad |= !(fabsf(x) <= 3.0e38f);
     f[q][lane] += to_fixed_j(x);
   }
-  __device__ __forceinline__ void flush(const PackView &v, int i, int s, int N) {
+  __device__ __forceinline__ void flush(const PackView &v, int i, int N) {
     long long *dst[7] = {v.hx + i, v.hy + i, v.hz + i, v.ej + i, v.ej + (size_t)N + i, v.ej + (size_t)2 * N + i,
                          v.ej + (size_t)3 * N + i};
 #pragma unroll
@@ -554,9 +581,12 @@ struct ISide {
       const long long x = f[q][lane];
       if (x) atomicAdd((unsigned long long *)dst[q], (unsigned long long)x);
     }
-    if (bad) atomicOr(&(v.ebuf ? v.sys_flags_alt : v.sys_flags)[s], SF_NONFINITE);
   }
 };
+// A non-finite partial (coincident atoms) marks its system.
+__device__ __forceinline__ void flush_bad(const PackView &v, bool bad, int s) {
+  if (bad) atomicOr(&(v.ebuf ? v.sys_flags_alt : v.sys_flags)[s], SF_NONFINITE);
+}
 
 // One tile's GB + LJ + Coulomb terms: the i side's sums of this lane's i
 // atom (io: force x, y, z, vdw, elec, pol, dE/da) and the j side's (jo,
@@ -595,9 +625,11 @@ __device__ __forceinline__ PairTileOut pair_tile(const ExactIn &v, const GbSetti
     io[1] -= cy;
     io[2] -= cz;
     const float c[7] = {cx, cy, cz, o.vdw, o.elec, o.epol, o.dedal * q.ib.w};
+    // (at t = 0 the source is this lane; plain additions, never contracted
+    // with the product a term may be)
     const int src = g8 | ((a - t) & 7);
 #pragma unroll
-    for (int k = 0; k < 7; k++) jo[k] += __shfl_sync(0xffffffffu, c[k], src);
+    for (int k = 0; k < 7; k++) jo[k] = __fadd_rn(jo[k], t == 0 ? c[k] : __shfl_sync(0xffffffffu, c[k], src));
   }
   PairTileOut o;
 #pragma unroll
@@ -607,14 +639,19 @@ __device__ __forceinline__ PairTileOut pair_tile(const ExactIn &v, const GbSetti
   }
   return o;
 }
-// The i-side inputs of this lane's atom of the tile's i-cluster.
-__device__ __forceinline__ void pair_i_side(const PackView &v, const TileInfo &ti, const SysParams *P, int lane,
-                                            PairTileIn &q) {
+// The i-side inputs of this lane's atom of the tile's i-cluster: what the
+// list build and the integrator wrote (with the fixed Born terms, kept in
+// ai_d), then the Born radius from the sum of the earlier phase.
+__device__ __forceinline__ void pair_i_static(const PackView &v, const TileInfo &ti, int lane, PairTileIn &q) {
   q.i = ti.a0 + (lane < ti.na ? lane : 0);
   q.ia = v.pq[2 * (size_t)q.i];
   q.ib = v.pq[2 * (size_t)q.i + 1];
   q.ip = v.prm[q.i];
-  q.ai_d = born_radius(v, *P, q.i);
+  q.ai_d = v.terms123[q.i];
+}
+__device__ __forceinline__ void pair_i_dyn(const PackView &v, double hec, double boff, PairTileIn &q) {
+  // k_born_finish's expression (born_radius; hec is -halfeconv)
+  q.ai_d = hec / (q.ai_d + (double)v.bsum[q.i] * kInvBornScale) + boff;
   q.ib.w = (float)q.ai_d;
 }
 // A tile's j records into this warp's slots, with each j atom's Born
@@ -642,34 +679,60 @@ __device__ __forceinline__ void pair_stage_j(const TileInfo &ti, const EvStage &
     sP[lane] = sP[lane + 8] = z;
   }
 }
-// The j side's sums of a tile over the i groups, added to the j atoms.
-__device__ __forceinline__ void pair_add_j(const PackView &v, const TileInfo &ti, int lane, float (&jacc)[7]) {
-  const int N = v.n_atoms;
+// Adds one FP32 partial of this lane to the fixed-point sum at p[at] when
+// `mine` (add_fixed without its branches: a zero adds nothing either way).
+__device__ __forceinline__ void add_fixed_if(bool mine, long long *p, float x, bool &bad) {
+  bad |= mine && !(fabsf(x) <= 3.0e38f);
+  const long long f = to_fixed_j(x);
+  if (mine && f) atomicAdd((unsigned long long *)p, (unsigned long long)f);
+}
+// The j side's sums of a tile over the i groups, added to the j atoms.  The
+// sums are (g0 + g1) + (g2 + g3) of the four groups' partials whichever group
+// forms them, so each exchange halves the quantities a group goes on with
+// (even groups keep 0-3, odd 4-6; then groups 0 and 2, 1 and 3 share those)
+// and a lane converts and adds two of its j atom's seven sums, not all seven
+// in the first group: 6 shuffles and 2 conversions a lane instead of 14 and 7.
+__device__ __forceinline__ void pair_add_j(const PackView &v, const TileInfo &ti, int lane, const float (&j)[7],
+                                           bool &bad) {
+  const int g = lane >> 3;
+  const bool odd = g & 1, high = g & 2;
+  float x[4];
 #pragma unroll
-  for (int k = 0; k < 7; k++) {
-    jacc[k] += __shfl_xor_sync(0xffffffffu, jacc[k], 8);
-    jacc[k] += __shfl_xor_sync(0xffffffffu, jacc[k], 16);
+  for (int k = 0; k < 4; k++) {
+    const float lo = j[k], hi = k < 3 ? j[4 + k] : 0.f;
+    const float other = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 8);
+    x[k] = __fadd_rn(odd ? hi : lo, other);
   }
-  if (lane < ti.nb) {
-    const int j = ti.b0 + lane;
-    add_fixed(v, &v.hx[j], jacc[0], ti.s);
-    add_fixed(v, &v.hy[j], jacc[1], ti.s);
-    add_fixed(v, &v.hz[j], jacc[2], ti.s);
+  float y[2];
 #pragma unroll
-    for (int k = 0; k < 4; k++) add_fixed(v, &v.ej[(size_t)k * N + j], jacc[3 + k], ti.s);
+  for (int k = 0; k < 2; k++) {
+    const float other = __shfl_xor_sync(0xffffffffu, high ? x[k] : x[2 + k], 16);
+    y[k] = __fadd_rn(high ? x[2 + k] : x[k], other);
   }
+  // group g holds quantities 4 odd + 2 high + {0, 1} (force x, y, z, vdw, elec,
+  // pol, dE/da; the eighth does not exist)
+  const int at = ti.b0 + (lane & 7);
+  const size_t N = (size_t)v.n_atoms;
+  long long *p0 = odd ? (high ? v.ej + 3 * N : v.ej + N) : (high ? v.hz : v.hx);
+  long long *p1 = odd ? v.ej + 2 * N : (high ? v.ej : v.hy);
+  const bool mine = (lane & 7) < ti.nb;
+  add_fixed_if(mine, p0 + at, y[0], bad);
+  add_fixed_if(mine && !(odd && high), p1 + at, y[1], bad);
 }
 
-template <bool LEAN>
-__device__ __forceinline__ void phase_pair(const PackView &v, int warp, int lane, float4 (*sA)[16],
-                                           float4 (*sB)[16], float4 (*sP)[16], long long (*sI)[7][32],
-                                           bool early) {
+// `wait` runs between the static loads of the first tile (its records, its
+// i side, the system's settings) and the first read of what the earlier
+// phase wrote; false ends the phase.
+template <bool LEAN, class Wait>
+__device__ __forceinline__ bool phase_pair(const PackView &v, int blocks, int warp, int lane, float4 (*sA)[16],
+                                           float4 (*sB)[16], float4 (*sP)[16], long long (*sI)[7][32], Wait wait) {
   int e, e1;
-  ev_range(v.tile_count[0], warp, e, e1);
+  ev_range(v.tile_count[0], blocks, warp, e, e1);
   const int first = e;
   const int N = v.n_atoms;
   const int g8 = lane & ~7, a = lane & 7;
   int a0 = -1, s_cur = -1, na = 0, s_i = 0, nd = 0;
+  bool jbad = false;  // a non-finite sum of a j atom
   ISide acc;
   acc.f = sI[warp];
   acc.lane = lane;
@@ -681,29 +744,43 @@ __device__ __forceinline__ void phase_pair(const PackView &v, int warp, int lane
   const SysParams *P = nullptr;
   double hec = 0.0, boff = 0.0;  // -halfeconv and the Born radius offset
   GbSettings gs;
+  auto settings = [&](int s) {
+    s_cur = s;
+    P = &v.sp[s];
+    gs.load(*P);
+    hec = -P->halfeconv_d;
+    boff = P->born_offset_d;
+  };
   const ExactIn xin = exact_in(v);
   EvWalk<2> walk;
   walk.start_static(v, lane, e, e1);
-  if (early) griddep_wait();
+  if (e < e1) {
+    const TileInfo ti = tile_info(walk.nx.m);
+    pair_i_static(v, ti, lane, q);
+    settings(ti.s);
+    a0 = ti.a0;
+    na = ti.na;
+    s_i = ti.s;
+  }
+  if (!wait()) return false;
   walk.start_dyn(v, lane);
+  if (e < e1) pair_i_dyn(v, hec, boff, q);
+#pragma unroll 1
   for (; e < e1; e++) {
     int te;
     const EvStage cur = walk.next(v, lane, te);
     const TileInfo ti = tile_info(cur.m);
-    if (ti.s != s_cur) {
-      s_cur = ti.s;
-      P = &v.sp[ti.s];
-      gs.load(*P);
-      hec = -P->halfeconv_d;
-      boff = P->born_offset_d;
-    }
     if (ti.a0 != a0) {
-      if (lane < na) acc.flush(v, q.i, s_i, N);
+      flush_bad(v, jbad || (lane < na && acc.bad), s_i);
+      if (lane < na) acc.flush(v, q.i, N);
       acc.clear();
+      jbad = false;
       a0 = ti.a0;
       na = ti.na;
       s_i = ti.s;
-      pair_i_side(v, ti, P, lane, q);
+      pair_i_static(v, ti, lane, q);
+      if (ti.s != s_cur) settings(ti.s);
+      pair_i_dyn(v, hec, boff, q);
     }
     q.b0 = ti.b0;
     pair_stage_j(ti, cur, lane, hec, boff, sA[warp], sB[warp], sP[warp]);
@@ -715,25 +792,25 @@ __device__ __forceinline__ void phase_pair(const PackView &v, int warp, int lane
     if (__any_sync(0xffffffffu, band)) {
       defer_tile(v, lane, first, nd, e);
     } else {
-      pair_add_j(v, ti, lane, o.jo);
+      pair_add_j(v, ti, lane, o.jo, jbad);
 #pragma unroll
       for (int k = 0; k < 7; k++) acc.add(k, o.io[k]);
     }
     __syncwarp();
   }
-  if (lane < na) acc.flush(v, q.i, s_i, N);
+  flush_bad(v, jbad || (lane < na && acc.bad), s_i);
+  if (lane < na) acc.flush(v, q.i, N);
   if (v.defer_stats && lane == 0 && nd) atomicAdd(&v.defer_stats[1], nd);
   // the deferred tiles in the careful form; their i sums go to memory at once
   __syncwarp();
+#pragma unroll 1
   for (int k = 0; k < nd; k++) {
     const int t = v.defer_list[first + k];
     const EvStage cur = ev_stage_one<2>(v, t, lane);
     const TileInfo ti = tile_info(cur.m);
-    P = &v.sp[ti.s];
-    gs.load(*P);
-    hec = -P->halfeconv_d;
-    boff = P->born_offset_d;
-    pair_i_side(v, ti, P, lane, q);
+    settings(ti.s);
+    pair_i_static(v, ti, lane, q);
+    pair_i_dyn(v, hec, boff, q);
     q.b0 = ti.b0;
     pair_stage_j(ti, cur, lane, hec, boff, sA[warp], sB[warp], sP[warp]);
     const unsigned rows = rot8(cur.row, a);
@@ -741,13 +818,16 @@ __device__ __forceinline__ void phase_pair(const PackView &v, int warp, int lane
     __syncwarp();
     bool band = false;
     PairTileOut o = pair_tile<true, LEAN>(xin, gs, P, q, sA[warp], sB[warp], sP[warp], rows, xrows, brows, a, g8, band);
-    pair_add_j(v, ti, lane, o.jo);
     acc.clear();
+    jbad = false;
+    pair_add_j(v, ti, lane, o.jo, jbad);
 #pragma unroll
     for (int c = 0; c < 7; c++) acc.add(c, o.io[c]);
-    if (lane < ti.na) acc.flush(v, q.i, ti.s, N);
+    flush_bad(v, jbad || (lane < ti.na && acc.bad), ti.s);
+    if (lane < ti.na) acc.flush(v, q.i, N);
     __syncwarp();
   }
+  return true;
 }
 
 // ============================================================= phase C
@@ -820,9 +900,9 @@ __device__ __forceinline__ ChainTileOut chain_tile(const ExactIn &v, const Chain
     io[1] += cy;
     io[2] += cz;
     const int src = g8 | ((a - t) & 7);
-    jo[0] += __shfl_sync(0xffffffffu, -cx, src);
-    jo[1] += __shfl_sync(0xffffffffu, -cy, src);
-    jo[2] += __shfl_sync(0xffffffffu, -cz, src);
+    jo[0] = __fadd_rn(jo[0], t == 0 ? -cx : __shfl_sync(0xffffffffu, -cx, src));
+    jo[1] = __fadd_rn(jo[1], t == 0 ? -cy : __shfl_sync(0xffffffffu, -cy, src));
+    jo[2] = __fadd_rn(jo[2], t == 0 ? -cz : __shfl_sync(0xffffffffu, -cz, src));
   }
   ChainTileOut o;
 #pragma unroll
@@ -832,16 +912,16 @@ __device__ __forceinline__ ChainTileOut chain_tile(const ExactIn &v, const Chain
   }
   return o;
 }
-// The i-side inputs of this lane's atom of the tile's i-cluster.
-__device__ __forceinline__ const SysParams *chain_i_side(const PackView &v, const TileInfo &ti, int lane,
-                                                         ChainTileIn &q) {
-  const int N = v.n_atoms;
+// The i-side inputs of this lane's atom of the tile's i-cluster: what is older
+// than the evaluation, then the chain weight from the earlier phases' sums.
+__device__ __forceinline__ const SysParams *chain_i_static(const PackView &v, const TileInfo &ti, int lane,
+                                                           ChainTileIn &q) {
   q.i = ti.a0 + (lane < ti.na ? lane : 0);
   q.ia = v.pq[2 * (size_t)q.i];
   q.ib = v.pq[2 * (size_t)q.i + 1];
   const float4 pi = v.prm[q.i];
+  q.ic = make_float4(pi.z, pi.w, 0.f, 0.f);
   const SysParams *P = &v.sp[ti.s];
-  q.ic = make_float4(pi.z, pi.w, chain_weight(*P, v.born_d[q.i], v.ej[(size_t)3 * N + q.i], q.ia.w), 0.f);
   q.s_hi = P->still2 * (1.f + 4e-6f);
   q.s_lo = P->still2 * (1.f - 4e-6f);
   q.invP5 = P->invP5;
@@ -849,6 +929,9 @@ __device__ __forceinline__ const SysParams *chain_i_side(const PackView &v, cons
   q.P4 = P->P4;
   q.still2_d = P->still2_d;
   return P;
+}
+__device__ __forceinline__ void chain_i_dyn(const PackView &v, const SysParams *P, ChainTileIn &q) {
+  q.ic.z = chain_weight(*P, v.born_d[q.i], v.ej[(size_t)3 * v.n_atoms + q.i], q.ia.w);
 }
 // A tile's j records (with each j atom's chain weight) into this warp's slots.
 __device__ __forceinline__ void chain_stage_j(const TileInfo &ti, const EvStage &cur, const SysParams *P, int lane,
@@ -860,34 +943,54 @@ __device__ __forceinline__ void chain_stage_j(const TileInfo &ti, const EvStage 
     sC[lane] = sC[lane + 8] = c;
   }
 }
-// A tile's forces: the j side summed over the i groups, and the i side.
-__device__ __forceinline__ void chain_add(const PackView &v, const TileInfo &ti, int lane, int i,
-                                          const ChainTileOut &o) {
-  float jo[3] = {o.jo[0], o.jo[1], o.jo[2]};
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    jo[c] += __shfl_xor_sync(0xffffffffu, jo[c], 8);
-    jo[c] += __shfl_xor_sync(0xffffffffu, jo[c], 16);
-  }
-  if (lane < ti.nb) {
-    const int j = ti.b0 + lane;
-    add_fixed(v, &v.hx[j], jo[0], ti.s);
-    add_fixed(v, &v.hy[j], jo[1], ti.s);
-    add_fixed(v, &v.hz[j], jo[2], ti.s);
-  }
-  if (lane < ti.na) {
-    add_fixed(v, &v.hx[i], o.io[0], ti.s);
-    add_fixed(v, &v.hy[i], o.io[1], ti.s);
-    add_fixed(v, &v.hz[i], o.io[2], ti.s);
-  }
+// The j side's forces of a tile, summed over the i groups as in pair_add_j
+// (even groups x and y, odd groups z; then group 0 x, group 2 y) and added to
+// the j atoms, one component a lane.
+__device__ __forceinline__ void chain_add_j(const PackView &v, const TileInfo &ti, int lane, const float (&j)[3],
+                                            bool &bad) {
+  const int g = lane >> 3;
+  const bool odd = g & 1, high = g & 2;
+  const float a = __fadd_rn(odd ? j[2] : j[0], __shfl_xor_sync(0xffffffffu, odd ? j[0] : j[2], 8));
+  const float b = __fadd_rn(j[1], __shfl_xor_sync(0xffffffffu, j[1], 8));
+  // an odd group holds z in a: both odd groups form the same sum
+  const float keep = odd ? a : (high ? b : a), give = odd ? a : (high ? a : b);
+  const float y = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, 16));
+  long long *p = odd ? v.hz : (high ? v.hy : v.hx);
+  add_fixed_if((lane & 7) < ti.nb && g != 3, p + ti.b0 + (lane & 7), y, bad);
 }
+// The i side's forces, fixed point per tile and added to memory when the
+// warp's range leaves the i-cluster (exact sums: the same bits).
+struct ChainISide {
+  long long f[3];
+  bool bad;
+  __device__ __forceinline__ void clear() {
+    f[0] = f[1] = f[2] = 0;
+    bad = false;
+  }
+  __device__ __forceinline__ void add(const float (&io)[3]) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      bad |= !(fabsf(io[c]) <= 3.0e38f);
+      f[c] += to_fixed_j(io[c]);
+    }
+  }
+  __device__ __forceinline__ void flush(const PackView &v, int i) {
+    if (f[0]) atomicAdd((unsigned long long *)&v.hx[i], (unsigned long long)f[0]);
+    if (f[1]) atomicAdd((unsigned long long *)&v.hy[i], (unsigned long long)f[1]);
+    if (f[2]) atomicAdd((unsigned long long *)&v.hz[i], (unsigned long long)f[2]);
+  }
+};
 
-__device__ __forceinline__ void phase_chain(const PackView &v, int warp, int lane, float4 (*sA)[16],
-                                            float4 (*sB)[16], float4 (*sC)[16], bool early) {
+template <class Wait>
+__device__ __forceinline__ bool phase_chain(const PackView &v, int blocks, int warp, int lane, float4 (*sA)[16],
+                                            float4 (*sB)[16], float4 (*sC)[16], Wait wait) {
   int q0, q1;
-  ev_range(v.tile_count[2], warp, q0, q1);
+  ev_range(v.tile_count[2], blocks, warp, q0, q1);  // (the still list is phase A's: complete)
   const int g8 = lane & ~7, a = lane & 7;
-  int a0 = -1, nd = 0;
+  int a0 = -1, na = 0, s_i = 0, nd = 0;
+  bool jbad = false;
+  ChainISide acc;
+  acc.clear();
   ChainTileIn q;
   q.ia = q.ib = q.ic = make_float4(0, 0, 0, 0);
   q.s_hi = q.s_lo = q.invP5 = q.piP5 = q.P4 = 0.f;
@@ -897,15 +1000,31 @@ __device__ __forceinline__ void phase_chain(const PackView &v, int warp, int lan
   const ExactIn xin = exact_in(v);
   EvWalk<4> walk;
   walk.start_static(v, lane, q0, q1);
-  if (early) griddep_wait();
+  if (q0 < q1) {
+    const TileInfo ti = tile_info(walk.nx.m);
+    P = chain_i_static(v, ti, lane, q);
+    a0 = ti.a0;
+    na = ti.na;
+    s_i = ti.s;
+  }
+  if (!wait()) return false;
   walk.start_dyn(v, lane);
+  if (q0 < q1) chain_i_dyn(v, P, q);
+#pragma unroll 1
   for (int k = q0; k < q1; k++) {
     int t;
     const EvStage cur = walk.next(v, lane, t);
     const TileInfo ti = tile_info(cur.m);
     if (ti.a0 != a0) {
+      flush_bad(v, jbad || (lane < na && acc.bad), s_i);
+      if (lane < na) acc.flush(v, q.i);
+      acc.clear();
+      jbad = false;
       a0 = ti.a0;
-      P = chain_i_side(v, ti, lane, q);
+      na = ti.na;
+      s_i = ti.s;
+      P = chain_i_static(v, ti, lane, q);
+      chain_i_dyn(v, P, q);
     }
     q.b0 = ti.b0;
     chain_stage_j(ti, cur, P, lane, sA[warp], sB[warp], sC[warp]);
@@ -913,37 +1032,50 @@ __device__ __forceinline__ void phase_chain(const PackView &v, int warp, int lan
     __syncwarp();
     bool band = false;
     const ChainTileOut o = chain_tile<false>(xin, q, sA[warp], sB[warp], sC[warp], rows, a, g8, band);
-    if (__any_sync(0xffffffffu, band))
+    if (__any_sync(0xffffffffu, band)) {
       defer_tile(v, lane, q0, nd, t);
-    else
-      chain_add(v, ti, lane, q.i, o);
+    } else {
+      chain_add_j(v, ti, lane, o.jo, jbad);
+      acc.add(o.io);
+    }
     __syncwarp();
   }
+  flush_bad(v, jbad || (lane < na && acc.bad), s_i);
+  if (lane < na) acc.flush(v, q.i);
   if (v.defer_stats && lane == 0 && nd) atomicAdd(&v.defer_stats[2], nd);
   // the deferred tiles in the careful form
   __syncwarp();
+#pragma unroll 1
   for (int k = 0; k < nd; k++) {
     const int t = v.defer_list[q0 + k];
     const EvStage cur = ev_stage_one<4>(v, t, lane);
     const TileInfo ti = tile_info(cur.m);
-    P = chain_i_side(v, ti, lane, q);
+    P = chain_i_static(v, ti, lane, q);
+    chain_i_dyn(v, P, q);
     q.b0 = ti.b0;
     chain_stage_j(ti, cur, P, lane, sA[warp], sB[warp], sC[warp]);
     const unsigned rows = rot8(cur.row & ~cur.x0, a);
     __syncwarp();
     bool band = false;
     const ChainTileOut o = chain_tile<true>(xin, q, sA[warp], sB[warp], sC[warp], rows, a, g8, band);
-    chain_add(v, ti, lane, q.i, o);
+    acc.clear();
+    jbad = false;
+    chain_add_j(v, ti, lane, o.jo, jbad);
+    acc.add(o.io);
+    flush_bad(v, jbad || (lane < ti.na && acc.bad), ti.s);
+    if (lane < ti.na) acc.flush(v, q.i);
     __syncwarp();
   }
+  return true;
 }
 
 // ============================================================= per-atom steps
 // Before phase A: zero what phase B adds into (and, first in an
 // evaluation, the forces and the record; ZeroFlags), as k_born_finish did.
-__device__ __forceinline__ void prologue_zero(const PackView &v, int zero) {
+__device__ __forceinline__ void prologue_zero(const PackView &v, int blocks, int zero) {
   const int N = v.n_atoms;
-  const int stride = gridDim.x * blockDim.x;
+  const int stride = blocks * blockDim.x;
+#pragma unroll 1
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
     for (int q = 0; q < 4; q++) v.ej[(size_t)q * N + i] = 0;
     if (zero) {
@@ -969,9 +1101,10 @@ __device__ __forceinline__ void prologue_zero(const PackView &v, int zero) {
   }
 }
 // After phase B (no phase-B reader of these): the Born radii.
-__device__ __forceinline__ void epilogue_radii(const PackView &v) {
+__device__ __forceinline__ void epilogue_radii(const PackView &v, int blocks) {
   const int N = v.n_atoms;
-  const int stride = gridDim.x * blockDim.x;
+  const int stride = blocks * blockDim.x;
+#pragma unroll 1
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
     const double a = born_radius(v, v.sp[v.sys_of[i]], i);
     v.born_d[i] = a;
@@ -980,9 +1113,10 @@ __device__ __forceinline__ void epilogue_radii(const PackView &v) {
 }
 // After phase C: the per-atom energies (k_gb_finish's values) and the
 // Born sums cleared for the next evaluation.
-__device__ __forceinline__ void epilogue_energies(const PackView &v) {
+__device__ __forceinline__ void epilogue_energies(const PackView &v, int blocks) {
   const int N = v.n_atoms;
-  const int stride = gridDim.x * blockDim.x;
+  const int stride = blocks * blockDim.x;
+#pragma unroll 1
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
     const SysParams &P = v.sp[v.sys_of[i]];
     const double dv = (double)v.ej[i] * kInvJScale;
@@ -1000,51 +1134,49 @@ __device__ __forceinline__ void epilogue_energies(const PackView &v) {
 }
 
 // ============================================================= the kernel
-// ph: which phases (1 A, 2 B, 4 C); more than one needs a cooperative
-// launch.  One compiled kernel serves the single launch and the three
-// one-phase launches, so both forms run the same instructions and give the
-// same bits whatever the compiler's contraction and scheduling choices.
-// MINB: resident blocks per SM the register allocation must allow
-// (PDGPU_EV_BLOCKS, 4 or 5, picks the build at run time; 4 by default).
-// tile_count[2] is the still-list length, tile_count[3] the barrier / exit
-// counter; the last block out clears both.
-template <int MINB, bool LEAN>
-__global__ void __launch_bounds__(32 * kEvWarps, MINB) k_eval_tiles(PackView v, int zero, int ph) {
+// PH: which phases (1 A, 2 B, 4 C); more than one needs a cooperative
+// launch.  tile_count[2] is the still-list length, tile_count[3] the barrier /
+// exit counter; the last block out clears both.
+template <bool LEAN, int PH>
+__global__ void __launch_bounds__(32 * kEvWarps, kEvBlocks) k_eval_tiles(PackView v, int zero) {
   // a launch of phase B or C alone follows the launch of the phase before
   // it: it stages its first tiles while that one still runs, and waits for
   // it (griddep_wait) before it reads anything the evaluation writes
-  const bool early = ph == 2 || ph == 4;
+  constexpr int ph = PH;
+  constexpr bool early = ph == 2 || ph == 4;
   if (!early) PDGPU_DEP_ENTRY();
-  if (v.flags[F_NL_OVERFLOW]) return;
+  const int G = ev_active(v);
+  if (v.flags[F_NL_OVERFLOW] || (int)blockIdx.x >= G) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __shared__ float4 s0[kEvWarps][16], s1[kEvWarps][16], s2[kEvWarps][16];
   __shared__ long long si[kEvWarps][7][32];  // phase B's i-side sums
   unsigned *ctr = reinterpret_cast<unsigned *>(&v.tile_count[3]);
-  const unsigned G = gridDim.x;
   unsigned passed = 0;  // barriers this launch has crossed
   if (ph & 1) {
-    prologue_zero(v, zero);
-    phase_born(v, warp, lane, s0, s1, s2);
+    prologue_zero(v, G, zero);
+    phase_born(v, G, warp, lane, s0, s1, s2);
   }
-  if ((ph & 1) && (ph & 6)) {
-    if (!grid_barrier(ctr, G * ++passed, v.flags)) return;
-  }
+  // phases B and C load their first tiles' older records, then wait for the
+  // phase before: a grid barrier in the cooperative launch, the previous
+  // launch's end otherwise
+  auto wait = [&](bool barrier) {
+    if (barrier) return grid_barrier(ctr, (unsigned)G * ++passed, v.flags);
+    if (early) griddep_wait();
+    return true;
+  };
   if (ph & 2) {
-    phase_pair<LEAN>(v, warp, lane, s0, s1, s2, si, early);
-    epilogue_radii(v);
-  }
-  if ((ph & 2) && (ph & 4)) {
-    if (!grid_barrier(ctr, G * ++passed, v.flags)) return;
+    if (!phase_pair<LEAN>(v, G, warp, lane, s0, s1, s2, si, [&] { return wait(ph & 1); })) return;
+    epilogue_radii(v, G);
   }
   if (ph & 4) {
-    phase_chain(v, warp, lane, s0, s1, s2, early);
-    epilogue_energies(v);
+    if (!phase_chain(v, G, warp, lane, s0, s1, s2, [&] { return wait(ph & 2); })) return;
+    epilogue_energies(v, G);
     // the last block out clears the still list and the counter
     __syncthreads();
     if (threadIdx.x == 0) {
       __threadfence();
       const unsigned prev = atomicAdd(ctr, 1u);
-      if (prev == G * (passed + 1) - 1) {
+      if (prev == (unsigned)G * (passed + 1) - 1) {
         v.tile_count[2] = 0;
         atomicExch(ctr, 0u);
       }
@@ -1073,25 +1205,14 @@ static int lean_allowed() {
   return w;
 }
 
-static int ev_minb() {
-  static int m = 0;
-  if (!m) {
-    const char *s = getenv("PDGPU_EV_BLOCKS");
-    m = (s && s[0] == '5') ? 5 : 4;
-  }
-  return m;
-}
-
 // Resident blocks of the evaluation kernel on this device (the grid of its
-// cooperative launch), and no more warps than a pack can have tiles.
+// launches; the one-phase builds keep at least as many resident), and no more
+// warps than a pack can have tiles.
 int eval_tiles_grid(long long tile_cap) {
   int dev = 0, sms = 148, occ = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (ev_minb() == 4)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_eval_tiles<4, false>, 32 * kEvWarps, 0);
-  else
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_eval_tiles<5, false>, 32 * kEvWarps, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_eval_tiles<false, 7>, 32 * kEvWarps, 0);
   const long long need = (tile_cap + kEvWarps - 1) / kEvWarps;
   return (int)std::max(1LL, std::min((long long)std::max(occ, 1) * sms, need));
 }
@@ -1120,12 +1241,13 @@ static cudaError_t launch_ev(int ph, const PackView &v, cudaStream_t st, int zer
   cfg.numAttrs = na;
   cudaError_t e;
   const bool lean = v.ev_lean && lean_allowed();
-  if (ev_minb() == 4)
-    e = lean ? cudaLaunchKernelEx(&cfg, k_eval_tiles<4, true>, v, zero, ph)
-                  : cudaLaunchKernelEx(&cfg, k_eval_tiles<4, false>, v, zero, ph);
-  else
-    e = lean ? cudaLaunchKernelEx(&cfg, k_eval_tiles<5, true>, v, zero, ph)
-                  : cudaLaunchKernelEx(&cfg, k_eval_tiles<5, false>, v, zero, ph);
+  auto go = [&](auto kernel) { return cudaLaunchKernelEx(&cfg, kernel, v, zero); };
+  switch (ph) {
+    case 1: e = lean ? go(k_eval_tiles<true, 1>) : go(k_eval_tiles<false, 1>); break;
+    case 2: e = lean ? go(k_eval_tiles<true, 2>) : go(k_eval_tiles<false, 2>); break;
+    case 4: e = lean ? go(k_eval_tiles<true, 4>) : go(k_eval_tiles<false, 4>); break;
+    default: e = lean ? go(k_eval_tiles<true, 7>) : go(k_eval_tiles<false, 7>); break;
+  }
   count_launch();
   return e;
 }

@@ -335,13 +335,11 @@ struct Pack {
       ene_pending[b] = false;
     }
   }
-  // evaluations may use the cooperative single-launch kernel (not for the
-  // request loop's jobs, whose streams run side by side).  Inside an MD
-  // step block the three-launch form is the default: its first phase starts
-  // while the bonded terms and the previous step's energy record still hold
-  // SMs, where a cooperative grid waits for all of its blocks to fit.
-  bool coop = true;
-  bool coop_md = false;
+  // the launch form of an evaluation on the tiles (pdgpu_eval_mode): three
+  // launches unless one cooperative launch was asked for (the default mode, 2,
+  // takes the faster form, which is the three launches at every size measured)
+  int eval_mode = 2;
+  bool coop = false, coop_md = false;  // single evaluations; MD step blocks
   ~Pack();
 };
 
