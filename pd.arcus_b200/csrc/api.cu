@@ -862,8 +862,6 @@ int pdgpu_zero_forces(pdgpu_ctx *c, int32_t sys) {
 }
 
 // ------------------------------------------------------------ kernels
-// enqueue a full list rebuild; when `size_check` the host reads the count
-// and grows the list buffer first (one synchronisation)
 }  // extern "C"
 // Grow the list buffer (stream-ordered) to hold `total` entries plus slack.
 int pdgpu::nlist_reserve(Pack &P, long long total, cudaStream_t st) {
@@ -885,21 +883,31 @@ int pdgpu::nlist_reserve(Pack &P, long long total, cudaStream_t st) {
 }
 extern "C" {
 
-static int nlist_enqueue(pdgpu_ctx *c, SysEntry *e, bool size_check) {
+// A rebuild with its host read-back: the first one of a pack sizes the
+// buffer between the count and the fill; later ones fill the buffer as it is
+// and read the count after it (one synchronisation, nothing waits for the
+// host in between), and only a list that outgrew it is filled again.
+static int nlist_enqueue(pdgpu_ctx *c, SysEntry *e) {
   Pack &P = *e->pack;
   PackView &v = P.v;
-  launch_nlist_count(P, c->st);
-  if (size_check) {
-    long long total = 0;
-    PDGPU_CUDA(cudaMemcpyAsync(&total, v.row_start + v.n_atoms, sizeof total, cudaMemcpyDeviceToHost, c->st));
-    int r = sync_check(c, "nlist count");
-    if (r) return r;
+  const bool sized = P.nl_total >= 0;
+  long long total = 0;
+  if (sized) {
+    PDGPU_CUDA(cudaMemsetAsync(v.flags + F_NL_OVERFLOW, 0, sizeof(int), c->st));
+    launch_nlist_rebuild(P, c->st);
+  } else {
+    launch_nlist_count(P, c->st);
+  }
+  PDGPU_CUDA(cudaMemcpyAsync(&total, v.row_start + v.n_atoms, sizeof total, cudaMemcpyDeviceToHost, c->st));
+  int r = sync_check(c, "nlist count");
+  if (r) return r;
+  if (!sized || total > v.nl_cap) {
     r = nlist_reserve(P, total, c->st);
     if (r) return r;
-    P.nl_total = total;
     PDGPU_CUDA(cudaMemsetAsync(v.flags + F_NL_OVERFLOW, 0, sizeof(int), c->st));
+    launch_nlist_fill(P, c->st);
   }
-  launch_nlist_fill(P, c->st);
+  P.nl_total = total;
   P.have_list = true;
   P.csr_stale = false;
   return PDGPU_OK;
@@ -922,8 +930,7 @@ static void rebuild_enqueue(Pack &P, cudaStream_t st) {
     launch_tiles_search(P.v, st);
     P.csr_stale = true;
   } else {
-    launch_nlist_count(P, st);
-    launch_nlist_fill(P, st);
+    launch_nlist_rebuild(P, st);
     P.csr_stale = false;
   }
 }
@@ -942,7 +949,7 @@ static int need_csr(pdgpu_ctx *c, SysEntry *e) {
   v.x = v.xs;
   v.y = v.xs + N;
   v.z = v.xs + 2 * N;
-  int r = nlist_enqueue(c, e, true);
+  int r = nlist_enqueue(c, e);
   v.x = x;
   v.y = y;
   v.z = z;
@@ -964,7 +971,7 @@ int pdgpu_nlist_build(pdgpu_ctx *c, int32_t sys) {
     rebuild_enqueue(P, c->st);
     return sync_check(c, "nlist_build");
   }
-  int r = nlist_enqueue(c, e, true);
+  int r = nlist_enqueue(c, e);
   if (r) return r;
   return sync_check(c, "nlist_build");
 }
@@ -1644,7 +1651,7 @@ static int md_run_impl(pdgpu_ctx *c, SysEntry *e, const pdgpu_md_params *p, int3
   // size the list once up front (one synchronisation); later rebuilds run
   // inside the step blocks and report overflow through a device flag
   if (!P.have_list || P.nl_total < 0) {
-    r = nlist_enqueue(c, e, true);
+    r = nlist_enqueue(c, e);
     if (r) return r;
   }
   if ((r = ready_pairs(c, e))) return r;
@@ -1762,7 +1769,7 @@ static int md_run_impl(pdgpu_ctx *c, SysEntry *e, const pdgpu_md_params *p, int3
       }
       if (flags[F_NL_OVERFLOW]) {
         // state untouched since the block start: grow the list and re-run
-        r = nlist_enqueue(c, e, true);
+        r = nlist_enqueue(c, e);
         if (r) return r;
         e->drop_graph();
         continue;
@@ -1837,7 +1844,7 @@ int pdgpu_minimise_run(pdgpu_ctx *c, int32_t sys, const pdgpu_min_params *p, int
   int every = p->UpdateNList;
   int r;
   if (!P.have_list || P.nl_total < 0) {
-    r = nlist_enqueue(c, e, true);
+    r = nlist_enqueue(c, e);
     if (r) return r;
   }
   if ((r = ready_pairs(c, e))) return r;
@@ -1894,7 +1901,7 @@ int pdgpu_minimise_run(pdgpu_ctx *c, int32_t sys, const pdgpu_min_params *p, int
         set_error("neighbour list kept overflowing during minimisation");
         return PDGPU_ERR_STATE;
       }
-      r = nlist_enqueue(c, e, true);  // sized rebuild at the current positions
+      r = nlist_enqueue(c, e);  // sized rebuild at the current positions
       if (r) return r;
       continue;
     }
@@ -2001,7 +2008,7 @@ int pdgpu_mc_run(pdgpu_ctx *c, int32_t sys, const pdgpu_mc_params *p, int32_t *a
   int r = default_seeds(c, e, p->Seed);
   if (r) return r;
   if (!P.have_list || P.nl_total < 0) {
-    if ((r = nlist_enqueue(c, e, true))) return r;
+    if ((r = nlist_enqueue(c, e))) return r;
   }
   if ((r = ready_pairs(c, e))) return r;
   // the starting state is the first base (and lowest) state
@@ -2048,7 +2055,7 @@ int pdgpu_mc_run(pdgpu_ctx *c, int32_t sys, const pdgpu_mc_params *p, int32_t *a
       int acc, done, ls;
       double low;
       mc_state_read(hs.data(), 0, &acc, &done, &low, &ls);
-      if ((r = nlist_enqueue(c, e, true))) return r;
+      if ((r = nlist_enqueue(c, e))) return r;
       PDGPU_CUDA(cudaMemsetAsync(v.flags + F_NL_OVERFLOW, 0, sizeof(int), c->st));
       step = done;
       continue;
@@ -2070,7 +2077,7 @@ int pdgpu_mc_run(pdgpu_ctx *c, int32_t sys, const pdgpu_mc_params *p, int32_t *a
   if ((r = sync_check(c, "mc_run final"))) return r;
   if ((r = barrier_check(c, P, flags))) return r;
   if (flags[F_NL_OVERFLOW]) {  // the final state's list: sized, then evaluated again
-    if ((r = nlist_enqueue(c, e, true))) return r;
+    if ((r = nlist_enqueue(c, e))) return r;
     calc_forces_enqueue(c->st, e, true, ws);
     if ((r = sync_check(c, "mc_run final"))) return r;
   }

@@ -377,6 +377,9 @@ void launch_zero(const PackView &v, cudaStream_t st);
 // neighbour list: build phases.  count -> (host may read total) -> fill
 void launch_nlist_count(Pack &p, cudaStream_t st);
 void launch_nlist_fill(Pack &p, cudaStream_t st);
+// count and fill together, into the list buffer as it is (F_NL_OVERFLOW when
+// it is too small; row_start[n_atoms] holds the entries needed)
+void launch_nlist_rebuild(Pack &p, cudaStream_t st);
 // GB.  zero: ZeroFlags bits; ZF_PAIRS zeroes the pair-force accumulators,
 // ZF_BONDED the bonded-force accumulators, ZF_RECORD the potential-energy
 // record and the system flags (together WorkSpace::zeroForces, so a step

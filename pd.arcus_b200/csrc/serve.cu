@@ -227,8 +227,7 @@ static void rebuild_pairs(Pack &P, cudaStream_t st) {
     launch_tiles_search(P.v, st);
     P.csr_stale = true;
   } else {
-    launch_nlist_count(P, st);
-    launch_nlist_fill(P, st);
+    launch_nlist_rebuild(P, st);
     P.csr_stale = false;
   }
 }
