@@ -17,7 +17,27 @@ struct pdgpu_ctx {
   std::map<int, std::unique_ptr<SysEntry>> sys;
   int next_id = 1;
   double last_ms = 0.0;
+  // A page-locked block for the small transfers of the calls (one at a time:
+  // a context is used by one host thread, and every call that uses the block
+  // ends with a synchronisation).  A pageable copy of a few KB costs about
+  // 10 us of driver staging; here the kernels read and write the block over
+  // the bus and the host copies from or to the caller's buffer.  Up to 256 KB
+  // (10,900 atoms): at 494 KB the host's copy costs what the driver's does.
+  void *pin = nullptr;
+  static constexpr size_t kPinBytes = 256 * 1024;
 };
+
+// The context's block when `bytes` fit and the caller's buffer is host memory
+// (anything else goes to the driver's copy, which reports it).
+static double *pinned(pdgpu_ctx *c, const void *user, size_t bytes) {
+  if (!c->pin || bytes > pdgpu_ctx::kPinBytes) return nullptr;
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, user) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return a.type == cudaMemoryTypeDevice ? nullptr : (double *)c->pin;
+}
 
 #define CHECK_CTX(c)                        \
   do {                                      \
@@ -60,6 +80,7 @@ static int get_sys(pdgpu_ctx *c, int id, bool device, SysEntry **out) {
   } while (0)
 
 
+static int small_out(pdgpu_ctx *c, void *dst, const void *src, size_t bytes, const char *what);
 static int sync_check(pdgpu_ctx *c, const char *what) {
   cudaError_t e = cudaStreamSynchronize(c->st);
   if (e != cudaSuccess) return cuda_fail(e, what);
@@ -77,8 +98,7 @@ static int barrier_check(pdgpu_ctx *c, pdgpu::Pack &P, const int *flags_host = n
   if (flags_host) {
     f = flags_host[F_BARRIER];
   } else if (P.v.tile_mode && P.coop) {  // (the three launches have no barrier)
-    PDGPU_CUDA(cudaMemcpyAsync(&f, P.v.flags + F_BARRIER, sizeof f, cudaMemcpyDeviceToHost, c->st));
-    int r = sync_check(c, "evaluation flags");
+    int r = small_out(c, &f, P.v.flags + F_BARRIER, sizeof f, "evaluation flags");
     if (r) return r;
   }
   if (!f) return PDGPU_OK;
@@ -260,12 +280,18 @@ int pdgpu_ctx_create(int device, pdgpu_ctx **out) {
     delete c;
     return cuda_fail(e, "cudaStreamCreate");
   }
+  // (without it the calls use pageable copies)
+  if (cudaHostAlloc(&c->pin, pdgpu_ctx::kPinBytes, cudaHostAllocMapped) != cudaSuccess) {
+    c->pin = nullptr;
+    cudaGetLastError();
+  }
   // the allocation-free list build's static scratch: loaded now, so a
   // caller that reserves its device memory after creating a context finds
   // the array already in place
   int r = noalloc_prepare_current_device();
   if (r) {
     cudaStreamDestroy(c->st);
+    if (c->pin) cudaFreeHost(c->pin);
     delete c;
     return r;
   }
@@ -280,6 +306,7 @@ int pdgpu_ctx_destroy(pdgpu_ctx *c) {
   c->sys.clear();
   cudaStreamSynchronize(c->st);
   cudaStreamDestroy(c->st);
+  if (c->pin) cudaFreeHost(c->pin);
   delete c;
   return PDGPU_OK;
 }
@@ -717,26 +744,55 @@ int pdgpu_perturb_torsions(pdgpu_ctx *c, int32_t sys, double sigma, uint64_t tri
 }
 
 // ------------------------------------------------------------ state
-// The caller's interleaved [n][3] buffer moves as one block to or from a
-// device staging array; the device reshuffles it (a page-locked caller
-// buffer is copied by DMA straight from or into its own memory).
-static int copy_soa_in(pdgpu_ctx *c, Pack &P, const double *xyz, double *X, double *Y, double *Z) {
-  const int n = P.v.n_atoms;
+}  // extern "C"
+// The caller's interleaved [n][3] buffer moves as one block, through the
+// context's page-locked block where it fits, else to or from a device staging
+// array (a page-locked caller buffer is copied by DMA straight from or into
+// its own memory); the device turns it.
+static int state_in(pdgpu_ctx *c, Pack &P, const double *xyz, const double *vel) {
+  const double *user = xyz ? xyz : vel;
+  const size_t bytes = sizeof(double) * 3 * (size_t)P.v.n_atoms;
+  const double *from = nullptr;
+  if (double *pin = pinned(c, user, bytes)) {
+    memcpy(pin, user, bytes);
+    from = pin;
+  } else {
+    int r = pack_ensure_stage(&P);
+    if (r) return r;
+    PDGPU_CUDA(cudaMemcpyAsync(P.stage, user, bytes, cudaMemcpyHostToDevice, c->st));
+    from = P.stage;
+  }
+  launch_state_in(P.v, xyz ? from : nullptr, vel ? from : nullptr, c->st);
+  return sync_check(c, xyz ? "set_positions" : "set_velocities");
+}
+// [n][3] out of the device: `form` enqueues the kernel that writes the
+// interleaved block to where it is given.
+template <typename Form>
+static int block_out(pdgpu_ctx *c, Pack &P, double *user, const char *what, Form form) {
+  const size_t bytes = sizeof(double) * 3 * (size_t)P.v.n_atoms;
+  if (double *pin = pinned(c, user, bytes)) {
+    form(pin);
+    int r = sync_check(c, what);
+    if (r) return r;
+    memcpy(user, pin, bytes);
+    return PDGPU_OK;
+  }
   int r = pack_ensure_stage(&P);
   if (r) return r;
-  PDGPU_CUDA(cudaMemcpyAsync(P.stage, xyz, sizeof(double) * 3 * (size_t)n, cudaMemcpyHostToDevice, c->st));
-  launch_aos_to_soa(P.stage, X, Y, Z, n, c->st);
+  form(P.stage);
+  PDGPU_CUDA(cudaMemcpyAsync(user, P.stage, bytes, cudaMemcpyDeviceToHost, c->st));
+  return sync_check(c, what);
+}
+// A few bytes of device memory read by the host.
+static int small_out(pdgpu_ctx *c, void *dst, const void *src, size_t bytes, const char *what) {
+  void *pin = bytes <= pdgpu_ctx::kPinBytes ? c->pin : nullptr;
+  PDGPU_CUDA(cudaMemcpyAsync(pin ? pin : dst, src, bytes, cudaMemcpyDeviceToHost, c->st));
+  int r = sync_check(c, what);
+  if (r) return r;
+  if (pin) memcpy(dst, pin, bytes);
   return PDGPU_OK;
 }
-static int copy_soa_out(pdgpu_ctx *c, Pack &P, double *xyz, const double *X, const double *Y,
-                        const double *Z) {
-  const int n = P.v.n_atoms;
-  int r = pack_ensure_stage(&P);
-  if (r) return r;
-  launch_soa_to_aos(P.stage, X, Y, Z, n, c->st);
-  PDGPU_CUDA(cudaMemcpyAsync(xyz, P.stage, sizeof(double) * 3 * (size_t)n, cudaMemcpyDeviceToHost, c->st));
-  return sync_check(c, "copy out");
-}
+extern "C" {
 
 int pdgpu_set_positions(pdgpu_ctx *c, int32_t sys, const double *xyz) {
   CHECK_CTX(c);
@@ -745,11 +801,7 @@ int pdgpu_set_positions(pdgpu_ctx *c, int32_t sys, const double *xyz) {
     set_error("xyz is NULL");
     return PDGPU_ERR_ARG;
   }
-  Pack &P = *e->pack;
-  int r = copy_soa_in(c, P, xyz, P.v.x, P.v.y, P.v.z);
-  if (r) return r;
-  launch_pack_positions(P.v, c->st);
-  return sync_check(c, "set_positions");
+  return state_in(c, *e->pack, xyz, nullptr);
 }
 int pdgpu_get_positions(pdgpu_ctx *c, int32_t sys, double *xyz) {
   CHECK_CTX(c);
@@ -758,8 +810,9 @@ int pdgpu_get_positions(pdgpu_ctx *c, int32_t sys, double *xyz) {
     set_error("xyz is NULL");
     return PDGPU_ERR_ARG;
   }
-  Pack &P = *e->pack;
-  return copy_soa_out(c, P, xyz, P.v.x, P.v.y, P.v.z);
+  const PackView &v = e->pack->v;
+  return block_out(c, *e->pack, xyz, "get_positions",
+                   [&](double *to) { launch_soa_to_aos(to, v.x, v.y, v.z, v.n_atoms, c->st); });
 }
 int pdgpu_set_velocities(pdgpu_ctx *c, int32_t sys, const double *v) {
   CHECK_CTX(c);
@@ -768,10 +821,7 @@ int pdgpu_set_velocities(pdgpu_ctx *c, int32_t sys, const double *v) {
     set_error("v is NULL");
     return PDGPU_ERR_ARG;
   }
-  Pack &P = *e->pack;
-  int r = copy_soa_in(c, P, v, P.v.vx, P.v.vy, P.v.vz);
-  if (r) return r;
-  return sync_check(c, "set_velocities");
+  return state_in(c, *e->pack, nullptr, v);
 }
 int pdgpu_get_velocities(pdgpu_ctx *c, int32_t sys, double *v) {
   CHECK_CTX(c);
@@ -780,8 +830,9 @@ int pdgpu_get_velocities(pdgpu_ctx *c, int32_t sys, double *v) {
     set_error("v is NULL");
     return PDGPU_ERR_ARG;
   }
-  Pack &P = *e->pack;
-  return copy_soa_out(c, P, v, P.v.vx, P.v.vy, P.v.vz);
+  const PackView &w = e->pack->v;
+  return block_out(c, *e->pack, v, "get_velocities",
+                   [&](double *to) { launch_soa_to_aos(to, w.vx, w.vy, w.vz, w.n_atoms, c->st); });
 }
 
 int pdgpu_get_forces(pdgpu_ctx *c, int32_t sys, double *f) {
@@ -792,11 +843,8 @@ int pdgpu_get_forces(pdgpu_ctx *c, int32_t sys, double *f) {
     return PDGPU_ERR_ARG;
   }
   Pack &P = *e->pack;
-  int r = pack_ensure_stage(&P);
-  if (r) return r;
-  launch_forces_out(P.v, consts().N_per_kcalmolA, P.stage, c->st);
-  PDGPU_CUDA(cudaMemcpyAsync(f, P.stage, sizeof(double) * 3 * (size_t)P.v.n_atoms, cudaMemcpyDeviceToHost, c->st));
-  return sync_check(c, "get_forces");
+  return block_out(c, P, f, "get_forces",
+                   [&](double *to) { launch_forces_out(P.v, consts().N_per_kcalmolA, to, c->st); });
 }
 
 int pdgpu_get_born_radii(pdgpu_ctx *c, int32_t sys, double *born) {
@@ -846,8 +894,7 @@ int pdgpu_get_energies(pdgpu_ctx *c, int32_t sys, double *ene, int32_t n) {
   static_assert(E_COUNT == PDGPU_ENE_COUNT, "energy record layout");
   Pack &P = *e->pack;
   std::vector<double> tmp((size_t)E_COUNT * S);
-  PDGPU_CUDA(cudaMemcpyAsync(tmp.data(), P.v.ene, sizeof(double) * tmp.size(), cudaMemcpyDeviceToHost, c->st));
-  int r = sync_check(c, "get_energies");
+  int r = small_out(c, tmp.data(), P.v.ene, sizeof(double) * tmp.size(), "get_energies");
   if (r) return r;
   double J = consts().J_per_kcalmol;
   for (size_t k = 0; k < tmp.size(); k++) ene[k] = tmp[k] * J;
@@ -898,8 +945,7 @@ static int nlist_enqueue(pdgpu_ctx *c, SysEntry *e) {
   } else {
     launch_nlist_count(P, c->st);
   }
-  PDGPU_CUDA(cudaMemcpyAsync(&total, v.row_start + v.n_atoms, sizeof total, cudaMemcpyDeviceToHost, c->st));
-  int r = sync_check(c, "nlist count");
+  int r = small_out(c, &total, v.row_start + v.n_atoms, sizeof total, "nlist count");
   if (r) return r;
   if (!sized || total > v.nl_cap) {
     r = nlist_reserve(P, total, c->st);
@@ -1192,20 +1238,28 @@ int pdgpu_gb_energies(pdgpu_ctx *c, int32_t sys) {
   int r = need_csr(c, e);
   if (r) return r;
   // calcEnergies: radii, FF_NonBonded::calcEnergies at Dielectric =
-  // DielectricSolute (gbff.cpp:44), then calcBornEnergy
+  // DielectricSolute (gbff.cpp:44), then calcBornEnergy.  The settings move
+  // to the device and back only where that dielectric is not the system's own
+  // already (the components' setup makes it so).
   const int S = e->nsys();
-  std::vector<SysParams> saved = P.sp;
-  for (int s = 0; s < S; s++) {
-    pdgpu_ff_params q = e->members[s]->params;
-    q.Dielectric = q.DielectricSolute;
-    pack_set_params(&P, s, q);
+  bool own = true;
+  for (int s = 0; s < S; s++) own = own && e->members[s]->params.Dielectric == e->members[s]->params.DielectricSolute;
+  std::vector<SysParams> saved;
+  if (!own) {
+    saved = P.sp;
+    for (int s = 0; s < S; s++) {
+      pdgpu_ff_params q = e->members[s]->params;
+      q.Dielectric = q.DielectricSolute;
+      pack_set_params(&P, s, q);
+    }
+    PDGPU_CUDA(cudaMemcpyAsync((void *)P.v.sp, P.sp.data(), sizeof(SysParams) * S, cudaMemcpyHostToDevice, c->st));
   }
-  PDGPU_CUDA(cudaMemcpyAsync((void *)P.v.sp, P.sp.data(), sizeof(SysParams) * S, cudaMemcpyHostToDevice, c->st));
   launch_born_radii(P.v, c->st);
   launch_nonbonded(P.v, c->st, P.sp[0].elec_mode);
   launch_born_energy(P.v, c->st);
   launch_energy(P.v, c->st, EM_PAIR_NB | EM_BORN_ENERGY);
   r = sync_check(c, "gb_energies");
+  if (own) return r;
   P.sp = saved;
   PDGPU_CUDA(cudaMemcpyAsync((void *)P.v.sp, P.sp.data(), sizeof(SysParams) * S, cudaMemcpyHostToDevice, c->st));
   int r2 = sync_check(c, "gb_energies");
@@ -1256,8 +1310,7 @@ static int lcpo_ready(pdgpu_ctx *c, SysEntry *e) {
 }
 static int lcpo_done(pdgpu_ctx *c, SysEntry *e, const char *what) {
   int flag = 0;
-  PDGPU_CUDA(cudaMemcpyAsync(&flag, e->pack->v.flags + F_LCPO_CAND, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-  int r = sync_check(c, what);
+  int r = small_out(c, &flag, e->pack->v.flags + F_LCPO_CAND, sizeof(int), what);
   if (r) return r;
   if (flag) {
     set_error(kLcpoCandMsg);
@@ -1297,9 +1350,21 @@ int pdgpu_sasa_lcpo_get(pdgpu_ctx *c, int32_t sys, double *sasa, double *deriv) 
     return PDGPU_ERR_STATE;
   }
   const size_t N = (size_t)e->pack->v.n_atoms;
+  Pack &P = *e->pack;
+  double *pin = pinned(c, deriv ? deriv : sasa, 4 * sizeof(double) * N);
+  if (pin && deriv && sasa && !pinned(c, sasa, 0)) pin = nullptr;
+  if (pin) {  // [deriv | sasa]
+    if (deriv) launch_soa_to_aos(pin, lc.deriv, lc.deriv + N, lc.deriv + 2 * N, (int)N, c->st);
+    if (sasa)
+      PDGPU_CUDA(cudaMemcpyAsync(pin + 3 * N, lc.sasa, sizeof(double) * N, cudaMemcpyDeviceToHost, c->st));
+    int r = sync_check(c, "sasa_lcpo_get");
+    if (r) return r;
+    if (deriv) memcpy(deriv, pin, sizeof(double) * 3 * N);
+    if (sasa) memcpy(sasa, pin + 3 * N, sizeof(double) * N);
+    return PDGPU_OK;
+  }
   if (sasa) PDGPU_CUDA(cudaMemcpyAsync(sasa, lc.sasa, sizeof(double) * N, cudaMemcpyDeviceToHost, c->st));
   if (deriv) {  // interleaved on the device, one block copied
-    Pack &P = *e->pack;
     int r = pack_ensure_stage(&P);
     if (r) return r;
     launch_soa_to_aos(P.stage, lc.deriv, lc.deriv + N, lc.deriv + 2 * N, (int)N, c->st);

@@ -59,22 +59,13 @@ void launch_pack_positions(const PackView &v, cudaStream_t st) {
   if (v.n_atoms) PDGPU_LAUNCH(k_pack_positions, (v.n_atoms + 255) / 256, 256, 0, st, v);
 }
 
-// Interleaved [n][3] <-> three arrays, on the device: the state transfer
-// calls move one contiguous block between the caller's buffer and a device
-// staging array, with no host-side reshuffle.
-__global__ void k_aos_to_soa(const double *aos, double *X, double *Y, double *Z, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  X[i] = aos[3 * (size_t)i];
-  Y[i] = aos[3 * (size_t)i + 1];
-  Z[i] = aos[3 * (size_t)i + 2];
-}
+// Three arrays -> interleaved [n][3]: one thread per component, so the stores
+// are contiguous (the destination may be the context's page-locked block).
 __global__ void k_soa_to_aos(double *aos, const double *X, const double *Y, const double *Z, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  aos[3 * (size_t)i] = X[i];
-  aos[3 * (size_t)i + 1] = Y[i];
-  aos[3 * (size_t)i + 2] = Z[i];
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 3 * n) return;
+  const int i = t / 3, k = t - 3 * i;
+  aos[t] = (k == 0 ? X : (k == 1 ? Y : Z))[i];
 }
 // The forces of the handle in N, interleaved [n][3], as the caller gets them:
 // the integrator's sum (fixed-point scattered terms, FP64 pair forces, the
@@ -101,14 +92,26 @@ void launch_forces_out(const PackView &v, double scale, double *out, cudaStream_
   if (v.n_atoms) PDGPU_LAUNCH(k_forces_out, (3 * v.n_atoms + 255) / 256, 256, 0, st, v, scale, out);
 }
 
-// The MD state in and out of pdgpu_md_run_io in one launch each: positions
-// (with the pair-kernel records) and velocities from / to interleaved
-// [n][3] staging blocks (either may be absent).
-__global__ void k_state_in(PackView v, const double *X, const double *V) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+// The state from / to interleaved [n][3] blocks in one launch: positions (with
+// the pair-kernel records) and velocities, either may be absent.  The blocks
+// are device staging or the context's page-locked block, read and written
+// over the bus: contiguous accesses, turned through shared memory on the way
+// in.
+constexpr int kStateThreads = 128;
+__global__ void __launch_bounds__(kStateThreads) k_state_in(PackView v, const double *X, const double *V) {
+  __shared__ double sx[3 * kStateThreads], sv[3 * kStateThreads];
+  const size_t b = 3 * (size_t)blockIdx.x * kStateThreads, n3 = 3 * (size_t)v.n_atoms;
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    const size_t t = b + q * kStateThreads + threadIdx.x;
+    if (X && t < n3) sx[q * kStateThreads + threadIdx.x] = X[t];
+    if (V && t < n3) sv[q * kStateThreads + threadIdx.x] = V[t];
+  }
+  __syncthreads();
+  const int i = blockIdx.x * kStateThreads + threadIdx.x, l = 3 * threadIdx.x;
   if (i >= v.n_atoms) return;
   if (X) {
-    const double x = X[3 * (size_t)i], y = X[3 * (size_t)i + 1], z = X[3 * (size_t)i + 2];
+    const double x = sx[l], y = sx[l + 1], z = sx[l + 2];
     v.x[i] = x;
     v.y[i] = y;
     v.z[i] = z;
@@ -123,37 +126,27 @@ __global__ void k_state_in(PackView v, const double *X, const double *V) {
     v.xyzp[i] = make_double4(x, y, z, v.pv_d[i]);
   }
   if (V) {
-    v.vx[i] = V[3 * (size_t)i];
-    v.vy[i] = V[3 * (size_t)i + 1];
-    v.vz[i] = V[3 * (size_t)i + 2];
+    v.vx[i] = sv[l];
+    v.vy[i] = sv[l + 1];
+    v.vz[i] = sv[l + 2];
   }
 }
 __global__ void k_state_out(PackView v, double *X, double *V) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= v.n_atoms) return;
-  if (X) {
-    X[3 * (size_t)i] = v.x[i];
-    X[3 * (size_t)i + 1] = v.y[i];
-    X[3 * (size_t)i + 2] = v.z[i];
-  }
-  if (V) {
-    V[3 * (size_t)i] = v.vx[i];
-    V[3 * (size_t)i + 1] = v.vy[i];
-    V[3 * (size_t)i + 2] = v.vz[i];
-  }
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 3 * v.n_atoms) return;
+  const int i = t / 3, k = t - 3 * i;
+  if (X) X[t] = (k == 0 ? v.x : (k == 1 ? v.y : v.z))[i];
+  if (V) V[t] = (k == 0 ? v.vx : (k == 1 ? v.vy : v.vz))[i];
 }
 void launch_state_in(const PackView &v, const double *X, const double *V, cudaStream_t st) {
-  if (v.n_atoms) PDGPU_LAUNCH(k_state_in, (v.n_atoms + 255) / 256, 256, 0, st, v, X, V);
+  if (v.n_atoms)
+    PDGPU_LAUNCH(k_state_in, (v.n_atoms + kStateThreads - 1) / kStateThreads, kStateThreads, 0, st, v, X, V);
 }
 void launch_state_out(const PackView &v, double *X, double *V, cudaStream_t st) {
-  if (v.n_atoms) PDGPU_LAUNCH(k_state_out, (v.n_atoms + 255) / 256, 256, 0, st, v, X, V);
-}
-
-void launch_aos_to_soa(const double *aos, double *X, double *Y, double *Z, int n, cudaStream_t st) {
-  if (n > 0) PDGPU_LAUNCH(k_aos_to_soa, (n + 255) / 256, 256, 0, st, aos, X, Y, Z, n);
+  if (v.n_atoms) PDGPU_LAUNCH(k_state_out, (3 * v.n_atoms + 255) / 256, 256, 0, st, v, X, V);
 }
 void launch_soa_to_aos(double *aos, const double *X, const double *Y, const double *Z, int n, cudaStream_t st) {
-  if (n > 0) PDGPU_LAUNCH(k_soa_to_aos, (n + 255) / 256, 256, 0, st, aos, X, Y, Z, n);
+  if (n > 0) PDGPU_LAUNCH(k_soa_to_aos, (3 * n + 255) / 256, 256, 0, st, aos, X, Y, Z, n);
 }
 
 __global__ void k_zero(PackView v) {

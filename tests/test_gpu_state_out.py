@@ -27,3 +27,32 @@ def test_forces_out_at_block_edges(n, gpu_ctx):
     f_ref, _, _ = S.calc_forces(pos, *S.nlist(pos))
     assert rel_rms(ws.cur.f, f_ref) <= 1e-5
     ws.close()
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 10922, 10923])
+def test_state_through_the_block_and_past_it(n, gpu_ctx):
+    """Positions and velocities in and out around a block of the kernels and
+    around the size the page-locked block holds (256 KB: 10,922 atoms): the
+    same bits come back, one array at a time and through pdgpu_md_run_io with
+    no step to run."""
+    import ctypes
+
+    import pdgpu
+    from pdgpu import _abi as A
+    rng = np.random.default_rng(n)
+    x, v = rng.normal(0.0, 200.0, (n, 3)), rng.normal(0.0, 400.0, (n, 3))
+    arrays, meta = _system(x, np.arange(n) % 300)
+    ws, ff = build_workspace(arrays, meta, gpu_ctx)
+    ws.cur.p[:], ws.cur.v[:] = x, v
+    ws._push_positions()
+    ws._push_velocities()
+    ws.cur.p[:], ws.cur.v[:] = 0.0, 0.0
+    ws._pull_positions()
+    ws._pull_velocities()
+    assert np.array_equal(ws.cur.p, x) and np.array_equal(ws.cur.v, v)
+    xo, vo = np.zeros((n, 3)), np.zeros((n, 3))
+    p = pdgpu.md_params_default()
+    A.check(pdgpu.lib().pdgpu_md_run_io(ws.ctx.ptr, ws._sys, ctypes.byref(p), 0, 0, 0, A.dptr(v), A.dptr(x),
+                                        A.dptr(xo), A.dptr(vo), None))
+    assert np.array_equal(xo, v) and np.array_equal(vo, x)
+    ws.close()
