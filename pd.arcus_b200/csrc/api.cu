@@ -1384,8 +1384,9 @@ void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce) {
   step.imm = e->ws_step;
   calc_forces_enqueue(st, e, reduce, step);
 }
-void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepSrc step, int ebuf, int coop) {
+void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepSrc step, const EvalOpts &o) {
   Pack &P = *e->pack;
+  const int ebuf = o.ebuf;
   const bool bonded = has_bonded(P);
   const bool surf = P.v.lc.update > 0;
   const bool side = bonded || surf;
@@ -1412,7 +1413,7 @@ void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepS
     if (slow) P.wait_energy(st, ebuf ^ 1);
     PackView vb = P.v;
     vb.ebuf = ebuf;
-    launch_eval_tiles(vb, st, zero, coop < 0 ? P.coop : coop != 0);
+    launch_eval_tiles(vb, st, zero | (o.old_tiles ? ZF_OLD_TILES : 0), o.coop < 0 ? P.coop : o.coop != 0);
     P.last_ebuf = ebuf;
   } else {
     launch_born_radii(P.v, st, zero);
@@ -1425,7 +1426,10 @@ void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepS
   // FastMode off: FF_NonBonded::calcForces beside calcBornForces
   if (slow) launch_nonbonded(P.v, st, P.sp[0].elec_mode);
   if (side) cudaStreamWaitEvent(st, P.join, 0);
-  if (reduce) launch_energy(P.v, st, pair_energy_mode(P) | (bonded ? EM_BONDED : 0) | (surf ? EM_SURF : 0));
+  if (o.ctl) launch_min_dots(P.v, st, *o.ctl);
+  if (reduce)
+    launch_energy(P.v, st, pair_energy_mode(P) | (bonded ? EM_BONDED : 0) | (surf ? EM_SURF : 0), nullptr, nullptr,
+                  o.ctl);
 }
 extern "C" {
 
@@ -1550,7 +1554,11 @@ void pdgpu::md_step_enqueue(cudaStream_t st, SysEntry *e, const MDCoef &k, int q
   StepSrc step;
   step.p = e->step_dev;  // MolecularDynamics::run_core sets WorkSpace::Step = Step (md.cpp:214)
   const int b = (P.v.tile_mode && !P.slow()) ? (q & 1) : 0;  // this step's energy buffer
-  calc_forces_enqueue(st, e, false, step, b, P.coop_md ? 1 : 0);
+  EvalOpts o;
+  o.ebuf = b;
+  o.coop = P.coop_md ? 1 : 0;
+  o.old_tiles = q > 0;  // (a block's first step may follow the launch that made them)
+  calc_forces_enqueue(st, e, false, step, o);
   // the integrator writes the kinetic energies the previous step's record
   // reads: that record must be done
   P.wait_energy(st, b ^ 1);
@@ -1920,6 +1928,7 @@ int pdgpu_minimise_run(pdgpu_ctx *c, int32_t sys, const pdgpu_min_params *p, int
   // iterations the device actually took; every system still running takes
   // one step per iteration, and a finished system (converged, out of
   // steps, NaN) sits the rest out.
+  const MinCtl ctl = min_ctl(e->min_state, p->Algorithm, slope, strict, steps);
   const int counter0 = P.nlist_counter;
   int iter = 0, regrow = 0;
   std::vector<int> taken(S, 0);
@@ -1927,9 +1936,13 @@ int pdgpu_minimise_run(pdgpu_ctx *c, int32_t sys, const pdgpu_min_params *p, int
     int chunk = std::min(16, steps - iter);
     for (int q = 0; q < chunk; q++) {
       int cnt = counter0 + iter + q;
-      if (every > 0 && (cnt % every) == 0) rebuild_enqueue(P, c->st);
-      calc_forces_enqueue(c->st, e, true, min_step_src(e->min_state, false));
-      launch_min_step(v, c->st, e->min_state, p->Algorithm, slope, strict, p->StepSize, steps);
+      const bool rebuild = every > 0 && (cnt % every) == 0;
+      if (rebuild) rebuild_enqueue(P, c->st);
+      EvalOpts o;
+      o.old_tiles = !rebuild && q > 0;
+      o.ctl = &ctl;
+      calc_forces_enqueue(c->st, e, true, min_step_src(e->min_state, false), o);
+      launch_min_update(v, c->st, ctl, p->StepSize);
     }
     int flags[F_COUNT];
     PDGPU_CUDA(cudaMemcpyAsync(flags, v.flags, sizeof flags, cudaMemcpyDeviceToHost, c->st));

@@ -24,7 +24,7 @@
 // 8.0, and it is the small systems' steps that wait for this record).
 #include <cuda_runtime.h>
 
-#include "internal.cuh"
+#include "minstep.cuh"
 
 namespace pdgpu {
 
@@ -54,7 +54,7 @@ __device__ __forceinline__ double chunk_sum(const double *p, int b, int e) {
 // hist: [step][sys][3] (epot, ekin, etot); step_dev[0] current step,
 // step_dev[1] first step of the run, step_dev[2] finished-system counter.
 __global__ void __launch_bounds__(kEnergyThreads) k_energy(PackView v, int mode, int C, double J2kcalmol,
-                                                           double *hist, int *step_dev) {
+                                                           double *hist, int *step_dev, MinCtl ctl) {
   // the ranges are fixed with the pack: read before the wait
   const int c = blockIdx.x, s = blockIdx.y, N = v.n_atoms;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energy(PackView v, int mode,
     }
     if (sflag & SF_NONFINITE) R[E_EPOT] = __longlong_as_double(0x7ff8000000000000LL);  // NaN
     if (!(R[E_EPOT] == R[E_EPOT])) atomicExch(&v.flags[F_NAN], 1);
+    if (ctl.ms) min_control(v, ctl.ms[s], ctl, R[E_EPOT]);
 #pragma unroll
     for (int k = 0; k < E_COUNT; k++) sE[k] = R[k];
   }
@@ -229,11 +230,12 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energy(PackView v, int mode,
   }
 }
 
-void launch_energy(const PackView &v, cudaStream_t st, int mode, double *hist, int *step_dev) {
+void launch_energy(const PackView &v, cudaStream_t st, int mode, double *hist, int *step_dev, const MinCtl *ctl) {
   if (!v.n_sys) return;
   const Consts &k = consts();
   int C = v.e_chunks;
-  PDGPU_LAUNCH_DEP(k_energy, dim3(C, v.n_sys), kEnergyThreads, 0, st, v, mode, C, k.J2kcal * k.Na, hist, step_dev);
+  PDGPU_LAUNCH_DEP(k_energy, dim3(C, v.n_sys), kEnergyThreads, 0, st, v, mode, C, k.J2kcal * k.Na, hist, step_dev,
+                   ctl ? *ctl : MinCtl());
 }
 
 }  // namespace pdgpu

@@ -18,8 +18,11 @@ void launch_md_step_impl(const PackView &v, cudaStream_t st, const MDCoef &c, co
 void launch_pair_counts(const PackView &v, cudaStream_t st, unsigned long long *out);
 void launch_ke_from_velocities(const PackView &v, cudaStream_t st);
 void launch_vel_init_impl(const PackView &v, cudaStream_t st, double temp, const unsigned long long *seeds);
-void launch_min_step(const PackView &v, cudaStream_t st, void *ms, int algorithm, double slope_kcal,
-                     double strict_kcal, double step_size, int nsteps);
+// a minimiser step after its forces: min_ctl gives the energy record the
+// control; the CG dot products run before it, the update after it
+MinCtl min_ctl(void *ms, int algorithm, double slope_kcal, double strict_kcal, int nsteps);
+void launch_min_dots(const PackView &v, cudaStream_t st, const MinCtl &c);
+void launch_min_update(const PackView &v, cudaStream_t st, const MinCtl &c, double step_size);
 void launch_min_finish(const PackView &v, cudaStream_t st);
 // where the LCPO term reads each system's WorkSpace::Step inside a
 // minimisation: the step being evaluated, or (last) the last step taken
@@ -171,8 +174,15 @@ bool has_bonded(const Pack &P);
 // chain rule, surface term; one energy reduction if reduce.  `step` is
 // where the surface term reads WorkSpace::Step (default: e->ws_step).
 void calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce);
-// (coop: -1 = the pack's single-evaluation launch form, else 0/1)
-void calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepSrc step, int ebuf = 0, int coop = -1);
+// coop: -1 = the pack's single-evaluation launch form, else 0/1.  old_tiles:
+// the launch before this evaluation did not make the tiles.  ctl: a minimiser
+// step's control, taken with the reduction.
+struct EvalOpts {
+  int ebuf = 0, coop = -1;
+  bool old_tiles = false;
+  const MinCtl *ctl = nullptr;
+};
+void calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepSrc step, const EvalOpts &o = EvalOpts());
 // one MD step: forces, integrator, energy record (+ step counter advance);
 // q = the step's index in its block (its energy buffer is q & 1 on tiles)
 void md_step_enqueue(cudaStream_t st, SysEntry *e, const MDCoef &k, int q);

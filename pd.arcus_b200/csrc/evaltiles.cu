@@ -152,8 +152,10 @@ struct EvStage {
 // only what the list build and the integrator wrote (the tile records,
 // coordinates, per-atom parameters); the dynamic part what the evaluation's
 // earlier phases wrote (the Born sums; the Born radii and dE/da sums).
+// (Of the static part, what the integrator did not write comes first: phase A
+// of a step without a rebuild reads that much before its wait.)
 template <int PH>
-__device__ __forceinline__ void ev_stage_static(const PackView &v, int t, int lane, EvStage &q) {
+__device__ __forceinline__ void ev_stage_old(const PackView &v, int t, int lane, EvStage &q) {
   q.row = tile_row(v, t, lane);
   q.x0 = q.x1 = 0;
   if (q.m.y >= 0) {
@@ -162,10 +164,15 @@ __device__ __forceinline__ void ev_stage_static(const PackView &v, int t, int la
   }
   if (lane <= (q.m.w & 7)) {
     const int j = q.m.x + lane;
-    q.a = v.pq[2 * (size_t)j];
-    q.b = v.pq[2 * (size_t)j + 1];
     q.c = v.prm[j];
     if (PH == 2) q.u = v.terms123[j];
+  }
+}
+__device__ __forceinline__ void ev_stage_xyz(const PackView &v, int lane, EvStage &q) {
+  if (lane <= (q.m.w & 7)) {
+    const int j = q.m.x + lane;
+    q.a = v.pq[2 * (size_t)j];
+    q.b = v.pq[2 * (size_t)j + 1];
   }
 }
 template <int PH>
@@ -181,15 +188,15 @@ __device__ __forceinline__ void ev_stage_dyn(const PackView &v, int lane, EvStag
 }
 template <int PH>
 __device__ __forceinline__ void ev_stage(const PackView &v, int t, int lane, EvStage &q) {
-  ev_stage_static<PH>(v, t, lane, q);
+  ev_stage_old<PH>(v, t, lane, q);
+  ev_stage_xyz(v, lane, q);
   ev_stage_dyn<PH>(v, lane, q);
 }
 // Walks a warp's tiles [e, e1) (PH 1, 2) or still-list entries (PH 4) with
 // the two-deep prefetch: next() returns the stage of the current tile and
-// its index, and issues the loads for the tiles after it.  start() is in
-// two parts: the static loads of the first items (which a launch may issue
-// before the earlier phases of its evaluation are done), then the dynamic
-// part of the first item's stage.
+// its index, and issues the loads for the tiles after it.  The start is in
+// parts: the loads of the first items that a launch may issue before the
+// launches before it are done, then the rest of the first item's stage.
 template <int PH>
 struct EvWalk {
   int e, e1;
@@ -199,14 +206,14 @@ struct EvWalk {
   __device__ __forceinline__ int tile_of(const PackView &v, int k) const {
     return PH == 4 ? v.still_list[k] : k;
   }
-  __device__ __forceinline__ void start_static(const PackView &v, int lane, int b, int end) {
+  __device__ __forceinline__ void start_old(const PackView &v, int lane, int b, int end) {
     e = b;
     e1 = end;
     t0 = t1 = t2 = 0;
     if (e < e1) {
       t0 = tile_of(v, e);
       nx.m = v.tile_meta[t0];
-      ev_stage_static<PH>(v, t0, lane, nx);
+      ev_stage_old<PH>(v, t0, lane, nx);
     }
     if (e + 1 < e1) {
       t1 = tile_of(v, e + 1);
@@ -214,12 +221,11 @@ struct EvWalk {
     }
     if (e + 2 < e1) t2 = tile_of(v, e + 2);
   }
+  __device__ __forceinline__ void start_xyz(const PackView &v, int lane) {
+    if (e < e1) ev_stage_xyz(v, lane, nx);
+  }
   __device__ __forceinline__ void start_dyn(const PackView &v, int lane) {
     if (e < e1) ev_stage_dyn<PH>(v, lane, nx);
-  }
-  __device__ __forceinline__ void start(const PackView &v, int lane, int b, int end) {
-    start_static(v, lane, b, end);
-    start_dyn(v, lane);
   }
   // the current item's stage and tile; advances the prefetch by one item
   __device__ __forceinline__ EvStage next(const PackView &v, int lane, int &tile) {
@@ -344,11 +350,10 @@ __device__ __forceinline__ BornTileOut born_tile(const ExactIn &v, const BornTil
   o.any = any;
   return o;
 }
-// The i-side inputs of atom i of the tile's i-cluster (this lane's).
-__device__ __forceinline__ void born_i_side(const PackView &v, const TileInfo &ti, int lane, BornTileIn &q) {
+// The i-side inputs of atom i of the tile's i-cluster (this lane's): the
+// parameters, then the position.
+__device__ __forceinline__ void born_i_old(const PackView &v, const TileInfo &ti, int lane, BornTileIn &q) {
   q.i = ti.a0 + (lane < ti.na ? lane : 0);
-  q.ia = v.pq[2 * (size_t)q.i];
-  q.ib = v.pq[2 * (size_t)q.i + 1];
   const float4 pi = v.prm[q.i];
   q.Ri = pi.z;
   q.Vi = pi.w;
@@ -359,6 +364,10 @@ __device__ __forceinline__ void born_i_side(const PackView &v, const TileInfo &t
   q.piP5 = P.piP5;
   q.P4s = P.P4 * (float)kBornScale;
   q.still2_d = P.still2_d;
+}
+__device__ __forceinline__ void born_i_xyz(const PackView &v, BornTileIn &q) {
+  q.ia = v.pq[2 * (size_t)q.i];
+  q.ib = v.pq[2 * (size_t)q.i + 1];
 }
 // A tile's j records into this warp's slots.
 __device__ __forceinline__ void born_stage_j(const TileInfo &ti, const EvStage &cur, int lane, float4 *sA,
@@ -376,8 +385,11 @@ __device__ __forceinline__ void born_add_j(const PackView &v, const TileInfo &ti
   if (lane < ti.nb && jacc) atomicAdd((unsigned long long *)&v.bsum[ti.b0 + lane], (unsigned long long)jacc);
 }
 
+// `wait` runs after the loads of what is older than the launch before (with
+// ZF_OLD_TILES: the tiles and the parameters).
+template <class Wait>
 __device__ __forceinline__ void phase_born(const PackView &v, int blocks, int warp, int lane, float4 (*sA)[16],
-                                           float4 (*sB)[16], float4 (*sC)[16]) {
+                                           float4 (*sB)[16], float4 (*sC)[16], Wait wait) {
   int e, e1;
   ev_range(v.tile_count[0], blocks, warp, e, e1);
   const int first = e;
@@ -393,7 +405,16 @@ __device__ __forceinline__ void phase_born(const PackView &v, int blocks, int wa
   int run0 = e;
   const ExactIn xin = exact_in(v);
   EvWalk<1> walk;
-  walk.start(v, lane, e, e1);
+  walk.start_old(v, lane, e, e1);
+  if (e < e1) {
+    const TileInfo ti = tile_info(walk.nx.m);
+    born_i_old(v, ti, lane, q);
+    a0 = ti.a0;
+    na = ti.na;
+  }
+  wait();
+  walk.start_xyz(v, lane);
+  if (e < e1) born_i_xyz(v, q);
   auto flush_near = [&](int upto) {
     // tiles [run0, upto) with their bits in `near`
     const int cnt = __popc(near);
@@ -416,7 +437,8 @@ __device__ __forceinline__ void phase_born(const PackView &v, int blocks, int wa
       acc_i = 0;
       a0 = ti.a0;
       na = ti.na;
-      born_i_side(v, ti, lane, q);
+      born_i_old(v, ti, lane, q);
+      born_i_xyz(v, q);
     }
     q.b0 = ti.b0;
     born_stage_j(ti, cur, lane, sA[warp], sB[warp], sC[warp]);
@@ -446,7 +468,8 @@ __device__ __forceinline__ void phase_born(const PackView &v, int blocks, int wa
     const int t = v.defer_list[first + k];
     const EvStage cur = ev_stage_one<1>(v, t, lane);
     const TileInfo ti = tile_info(cur.m);
-    born_i_side(v, ti, lane, q);
+    born_i_old(v, ti, lane, q);
+    born_i_xyz(v, q);
     q.b0 = ti.b0;
     born_stage_j(ti, cur, lane, sA[warp], sB[warp], sC[warp]);
     const unsigned rows = rot8(cur.row & ~cur.x0, a);
@@ -753,7 +776,8 @@ __device__ __forceinline__ bool phase_pair(const PackView &v, int blocks, int wa
   };
   const ExactIn xin = exact_in(v);
   EvWalk<2> walk;
-  walk.start_static(v, lane, e, e1);
+  walk.start_old(v, lane, e, e1);
+  walk.start_xyz(v, lane);
   if (e < e1) {
     const TileInfo ti = tile_info(walk.nx.m);
     pair_i_static(v, ti, lane, q);
@@ -999,7 +1023,8 @@ __device__ __forceinline__ bool phase_chain(const PackView &v, int blocks, int w
   const SysParams *P = nullptr;
   const ExactIn xin = exact_in(v);
   EvWalk<4> walk;
-  walk.start_static(v, lane, q0, q1);
+  walk.start_old(v, lane, q0, q1);
+  walk.start_xyz(v, lane);
   if (q0 < q1) {
     const TileInfo ti = tile_info(walk.nx.m);
     P = chain_i_static(v, ti, lane, q);
@@ -1078,7 +1103,7 @@ __device__ __forceinline__ void prologue_zero(const PackView &v, int blocks, int
 #pragma unroll 1
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
     for (int q = 0; q < 4; q++) v.ej[(size_t)q * N + i] = 0;
-    if (zero) {
+    if (zero & ZF_PAIRS) {
       if (zero & ZF_BONDED) {
         v.fx[i] = 0;
         v.fy[i] = 0;
@@ -1144,7 +1169,8 @@ __global__ void __launch_bounds__(32 * kEvWarps, kEvBlocks) k_eval_tiles(PackVie
   // it (griddep_wait) before it reads anything the evaluation writes
   constexpr int ph = PH;
   constexpr bool early = ph == 2 || ph == 4;
-  if (!early) PDGPU_DEP_ENTRY();
+  const bool old_tiles = ph == 1 && (zero & ZF_OLD_TILES);
+  if (!early && !old_tiles) PDGPU_DEP_ENTRY();
   const int G = ev_active(v);
   if (v.flags[F_NL_OVERFLOW] || (int)blockIdx.x >= G) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1153,8 +1179,10 @@ __global__ void __launch_bounds__(32 * kEvWarps, kEvBlocks) k_eval_tiles(PackVie
   unsigned *ctr = reinterpret_cast<unsigned *>(&v.tile_count[3]);
   unsigned passed = 0;  // barriers this launch has crossed
   if (ph & 1) {
-    prologue_zero(v, G, zero);
-    phase_born(v, G, warp, lane, s0, s1, s2);
+    phase_born(v, G, warp, lane, s0, s1, s2, [&] {
+      if (old_tiles) griddep_wait();
+      prologue_zero(v, G, zero);
+    });
   }
   // phases B and C load their first tiles' older records, then wait for the
   // phase before: a grid barrier in the cooperative launch, the previous

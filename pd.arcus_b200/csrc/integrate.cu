@@ -21,6 +21,7 @@
 #include <cstddef>
 
 #include "mdatom.cuh"
+#include "minstep.cuh"
 
 namespace pdgpu {
 
@@ -30,17 +31,22 @@ namespace pdgpu {
 // only, so they are drawn before the wait for the force passes (under a
 // programmatic dependent launch, beside the last pass's tail).  The step
 // counter is final by then: the step's launch waits on the event of the
-// energy record that advanced it, a full dependency.
+// energy record that advanced it, a full dependency.  The atom's mass,
+// velocity and position (the previous step's, complete before this step's
+// first phase passed its own wait) and the noise widths of its mass are ready
+// before the wait too; after it come the nine force loads and the update.
 __global__ void k_md_step(PackView v, MDDev d, const double *normals, const int *step_dev) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = i < v.n_atoms;
   const int step = !live ? 0 : step_dev ? *step_dev : d.c.step;
   double nr[6];
   const bool pre = live && !normals && md_draws_normals(v, d, step, i);
+  MDIn in;
+  if (live) md_load(v, d, i, in);
   if (pre) md_normals(v, d, step, i, nr);
   PDGPU_DEP_ENTRY();
   if (!live || v.flags[F_NL_OVERFLOW]) return;  // forces incomplete: keep the state, host re-plans
-  v.e_atom[(size_t)AE_KIN * v.n_atoms + i] = md_atom(v, d, normals, step, i, pre ? nr : nullptr);  // J
+  v.e_atom[(size_t)AE_KIN * v.n_atoms + i] = md_atom(v, d, normals, step, i, in, pre ? nr : nullptr);  // J
 }
 
 // Kinetic energies from the current velocities: every atom's (J) and each
@@ -119,17 +125,12 @@ __global__ void k_vel_scale(PackView v, double kB, double temp, double kcal2J_pe
 }
 
 // --------------------------------------------------------------- minimiser
-struct MinState {
-  double mult, old_energy, local_old, gamma, fmagold, fmagnew;
-  int step, breakcount, done, action;  // action: 0 step, 1 restore-and-skip, 2 restore-then-step
-  int taken, nan;
-  int last;  // the last step the loop evaluated (WorkSpace::Step when the loop ends)
-};
-
 // CG dot products: per (chunk, system) partials of fmagold = sum of.of and
 // fmagnew = sum (of-f).f into e_part slots 0 and 1; the last block of each
-// system adds them in a fixed order for k_min_control.
-__global__ void k_min_dots(PackView v, double N_per_unit, int C) {
+// system adds them in a fixed order into its state, before the energy record
+// whose last block takes the step's decision (min_control).
+__global__ void k_min_dots(PackView v, MinState *ms, double N_per_unit, int C) {
+  PDGPU_DEP_ENTRY();
   if (v.flags[F_NL_OVERFLOW]) return;
   const int c = blockIdx.x, s = blockIdx.y;
   int a0 = v.atom_off[s] + c * kReduceChunk, a1 = min(a0 + kReduceChunk, v.atom_off[s + 1]);
@@ -158,7 +159,7 @@ __global__ void k_min_dots(PackView v, double N_per_unit, int C) {
     part[(size_t)c * 10 + 1] = sb[0];
   }
   // the last block of the system adds the chunk partials (lanes strided over
-  // the chunks, then a fixed shuffle tree) into slots 2 and 3 of chunk 0
+  // the chunks, then a fixed shuffle tree)
   __shared__ int last;
   __threadfence();
   __syncthreads();
@@ -171,100 +172,25 @@ __global__ void k_min_dots(PackView v, double N_per_unit, int C) {
     double t = 0.0;
     for (int q = lane; q < C; q += 32) t += __ldcg(part + (size_t)q * 10 + warp);
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == 0) part[2 + warp] = t;
+    if (lane == 0) (warp == 0 ? ms[s].fmagold : ms[s].fmagnew) = t;
   }
   if (threadIdx.x == 0) v.e_done[s] = 0;
 }
 
-// One thread per system: the accept / restore decision of the step.
-// Energies here are kcal/mol; one joule per molecule (the reference's
-// "m_OldEnergy += 1" after a rejected SD step) is J_unit kcal/mol.
-__global__ void k_min_control(PackView v, MinState *ms, int algorithm, double slope_cutoff_kcal,
-                              double strictness_kcal, double J_unit, int nsteps, int C) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= v.n_sys) return;
-  MinState &m = ms[s];
-  if (algorithm == PDGPU_MIN_CONJUGATE_GRADIENTS && !v.flags[F_NL_OVERFLOW]) {
-    const double *o = v.e_part + (size_t)s * C * 10;  // totals of k_min_dots
-    m.fmagold = o[2];
-    m.fmagnew = o[3];
-  }
-  if (v.flags[F_NL_OVERFLOW]) {  // no valid forces this step: do nothing, retry
-    m.action = -1;
-    return;
-  }
-  if (m.done) {
-    m.action = -1;
-    return;
-  }
-  m.last = m.step;
-  double epot = v.ene[(size_t)s * E_COUNT + E_EPOT];
-  if (!(epot == epot)) {
-    m.nan = 1;
-    m.done = 1;
-    m.action = -1;
-    atomicExch(&v.flags[F_NAN], 1);
-    return;
-  }
-  if (m.step == 0) m.local_old = epot;
-  if (m.step > 0 && slope_cutoff_kcal > 0.0) {
-    double d = m.local_old - epot;
-    if (d >= 0.0 && d < slope_cutoff_kcal) m.breakcount++;
-    m.local_old = epot;
-  }
-  if (m.breakcount > 10) {
-    m.done = 1;
-    m.action = -1;
-    return;
-  }
-  if (algorithm == PDGPU_MIN_STEEPEST_DESCENT) {
-    if (m.step != 0) {
-      if (epot <= m.old_energy) {
-        m.mult *= 1.2;
-        m.old_energy = epot;
-        m.action = 0;  // save then step
-      } else {
-        m.mult *= 0.5 / 1.2;
-        m.old_energy += J_unit;
-        m.action = 1;  // restore, no step
-      }
-    } else {
-      m.old_energy = epot;
-      m.action = 0;
-    }
-  } else {
-    if (m.step != 0) {
-      if ((m.mult < 0.05 && (epot - m.old_energy) < strictness_kcal) || epot < m.old_energy) {
-        m.mult *= 1.2;
-        double g = m.fmagold != 0 ? m.fmagnew / m.fmagold : 0.0;
-        if (g < 0) g = 0;
-        m.gamma = g;
-        m.old_energy = epot;
-        m.action = 3;  // new direction, save, step
-      } else {
-        m.mult *= 0.5 / 1.2;
-        m.action = 2;  // restore positions, step along the old direction
-      }
-    } else {
-      m.old_energy = epot;
-      m.action = 4;  // first step: direction = force
-    }
-  }
-  m.step++;
-  m.taken = m.step;
-  if (m.step >= nsteps) m.done = 1;
-}
-
+// The step of every atom by its system's decision.  Positions and forces are
+// older than the energy record this launch follows (the forces were complete
+// before it), so they are read before the wait and only the decision after it.
 __global__ void k_min_update(PackView v, const MinState *ms, double N_per_unit, double step_size) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= v.n_atoms) return;
   int s = v.sys_of[i];
-  const MinState &m = ms[s];
-  int a = m.action;
-  if (a < 0) return;
   double f[3] = {force_N(v.fx[i], v.gx[i], v.hx[i]) * N_per_unit, force_N(v.fy[i], v.gy[i], v.hy[i]) * N_per_unit,
                  force_N(v.fz[i], v.gz[i], v.hz[i]) * N_per_unit};
   double p[3] = {v.x[i], v.y[i], v.z[i]};
+  PDGPU_DEP_ENTRY();
+  const MinState &m = ms[s];
+  const int a = m.action;
+  if (a < 0 || v.flags[F_NL_OVERFLOW]) return;  // (no valid forces: nothing moves, the host retries)
   double sc = step_size * m.mult;
   if (a == 0) {  // SD accept (or first step): save p, f; step along f
     v.ox[i] = p[0];
@@ -366,16 +292,25 @@ void launch_vel_init_impl(const PackView &v, cudaStream_t st, double temp, const
   PDGPU_LAUNCH(k_vel_scale, (v.n_atoms + 255) / 256, 256, 0, st, v, k.kB, temp, k.kcal2J / k.Na);
   launch_ke_from_velocities(v, st);
 }
-void launch_min_step(const PackView &v, cudaStream_t st, void *ms, int algorithm, double slope_kcal,
-                     double strict_kcal, double step_size, int nsteps) {
+MinCtl min_ctl(void *ms, int algorithm, double slope_kcal, double strict_kcal, int nsteps) {
   const Consts &k = consts();
-  MinState *m = (MinState *)ms;
-  int C = v.e_chunks;
-  if (algorithm == PDGPU_MIN_CONJUGATE_GRADIENTS)
-    PDGPU_LAUNCH(k_min_dots, dim3(C, v.n_sys), 256, 0, st, v, k.N_per_kcalmolA, C);
-  PDGPU_LAUNCH(k_min_control, (v.n_sys + 127) / 128, 128, 0, st, v, m, algorithm, slope_kcal, strict_kcal,
-               k.J2kcal * k.Na, nsteps, C);
-  PDGPU_LAUNCH(k_min_update, (v.n_atoms + 63) / 64, 64, 0, st, v, m, k.N_per_kcalmolA, step_size);
+  MinCtl c;
+  c.ms = (MinState *)ms;
+  c.algorithm = algorithm;
+  c.nsteps = nsteps;
+  c.slope_kcal = slope_kcal;
+  c.strict_kcal = strict_kcal;
+  c.J_unit = k.J2kcal * k.Na;
+  return c;
+}
+void launch_min_dots(const PackView &v, cudaStream_t st, const MinCtl &c) {
+  if (c.algorithm != PDGPU_MIN_CONJUGATE_GRADIENTS) return;
+  const int C = v.e_chunks;
+  PDGPU_LAUNCH_DEP(k_min_dots, dim3(C, v.n_sys), 256, 0, st, v, c.ms, consts().N_per_kcalmolA, C);
+}
+void launch_min_update(const PackView &v, cudaStream_t st, const MinCtl &c, double step_size) {
+  if (v.n_atoms)
+    PDGPU_LAUNCH_DEP(k_min_update, (v.n_atoms + 63) / 64, 64, 0, st, v, c.ms, consts().N_per_kcalmolA, step_size);
 }
 void launch_min_finish(const PackView &v, cudaStream_t st) {
   if (v.n_atoms) PDGPU_LAUNCH(k_min_restore_best, (v.n_atoms + 255) / 256, 256, 0, st, v);

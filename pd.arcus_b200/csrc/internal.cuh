@@ -127,6 +127,14 @@ struct StepSrc {
   int imm = 0;
 };
 
+// A minimiser step's control, taken where its energy is formed (minstep.cuh).
+struct MinState;
+struct MinCtl {
+  MinState *ms = nullptr;  // [S]; NULL: no control
+  int algorithm = 0, nsteps = 0;
+  double slope_kcal = 0, strict_kcal = 0, J_unit = 0;
+};
+
 struct BondedTerms {
   int nb = 0, na = 0, nt = 0, ni = 0;
   const int *term_off = nullptr;  // [4*(S+1)]: bond, angle, torsion, improper ranges per system
@@ -383,7 +391,15 @@ void launch_nlist_rebuild(Pack &p, cudaStream_t st);
 // ZF_BONDED the bonded-force accumulators, ZF_RECORD the potential-energy
 // record and the system flags (together WorkSpace::zeroForces, so a step
 // needs no separate zeroing launch)
-enum ZeroFlags { ZF_PAIRS = 1, ZF_BONDED = 2, ZF_RECORD = 4 };
+enum ZeroFlags {
+  ZF_PAIRS = 1,
+  ZF_BONDED = 2,
+  ZF_RECORD = 4,
+  // not a zeroing: the tiles are older than the launch before this evaluation
+  // (a step without a rebuild), so its first phase may read them before its
+  // dependent-launch wait
+  ZF_OLD_TILES = 8
+};
 void launch_born_radii(const PackView &v, cudaStream_t st, int zero = 0);
 void launch_gb_pair(const PackView &v, cudaStream_t st);
 void launch_gb_chain(const PackView &v, cudaStream_t st);
@@ -433,8 +449,9 @@ void launch_lcpo_part(const PackView &v, cudaStream_t st, StepSrc step, bool ene
                       int part);
 // energies: per-atom / per-term energies into the per-system record
 // (mode = EnergyMode bits); hist/step_dev only with EM_RECORD
+// (ctl: a minimiser step's control on each system's energy)
 void launch_energy(const PackView &v, cudaStream_t st, int mode, double *hist = nullptr,
-                   int *step_dev = nullptr);
+                   int *step_dev = nullptr, const MinCtl *ctl = nullptr);
 // integrators / minimiser
 struct MDCoef {
   double dt, gamma, c0, c1, c2, varv, varr, crv, temp;

@@ -99,20 +99,45 @@ __device__ __forceinline__ void md_normals(const PackView &v, const MDDev &d, in
   six_normals(d.sys_seed[s], i - v.atom_off[s], step, nr);
 }
 
+// What an atom's step needs besides its force: its state and mass, and for
+// the Langevin update the quotients and noise widths of its mass.
+struct MDIn {
+  double m, im, sigmav, sigmar, vel[3], pos[3];
+  bool hyd;
+};
+__device__ __forceinline__ void md_load(const PackView &v, const MDDev &d, int i, MDIn &o) {
+  const MDCoef &c = d.c;
+  o.m = v.mass_si[i];
+  o.vel[0] = v.vx[i];
+  o.vel[1] = v.vy[i];
+  o.vel[2] = v.vz[i];
+  o.pos[0] = v.x[i];
+  o.pos[1] = v.y[i];
+  o.pos[2] = v.z[i];
+  o.hyd = d.is_h && d.is_h[i];
+  o.im = o.sigmav = o.sigmar = 0.0;
+  if (c.integrator == PDGPU_INTEGRATOR_LANGEVIN) {
+    o.im = 1.0 / o.m;
+    double kTdivm = d.kB * c.temp * o.im;
+    o.sigmav = sqrt(kTdivm * c.varv);
+    o.sigmar = sqrt(kTdivm * c.varr) * c.inv_gamma;
+  }
+}
+
 // Advance atom i by one step of the integrator in d.c at `step`; returns
 // its kinetic energy (J) at the point the reference measures it.  `pre`:
 // the atom's thermostat normals drawn already (md_normals), or NULL.
 __device__ __forceinline__ double md_atom(const PackView &v, const MDDev &d, const double *normals, int step,
-                                          int i, const double *pre = nullptr) {
+                                          int i, const MDIn &in, const double *pre = nullptr) {
   const MDCoef &c = d.c;
-  double m = v.mass_si[i];
+  const double m = in.m;
   double f[3] = {force_N(v.fx[i], v.gx[i], v.hx[i]) * d.N_per_unit, force_N(v.fy[i], v.gy[i], v.hy[i]) * d.N_per_unit,
                  force_N(v.fz[i], v.gz[i], v.hz[i]) * d.N_per_unit};
-  double vel[3] = {v.vx[i], v.vy[i], v.vz[i]};
-  double pos[3] = {v.x[i], v.y[i], v.z[i]};
+  double vel[3] = {in.vel[0], in.vel[1], in.vel[2]};
+  double pos[3] = {in.pos[0], in.pos[1], in.pos[2]};
   double t = c.dt;
   int integ = c.integrator;
-  bool hyd = d.is_h && d.is_h[i];
+  const bool hyd = in.hyd;
   bool langevin = integ == PDGPU_INTEGRATOR_LANGEVIN;
   if (langevin && c.gamma * t < 0.00001) integ = PDGPU_INTEGRATOR_VELOCITY_VERLET, langevin = false;
   bool vv_like = integ == PDGPU_INTEGRATOR_VELOCITY_VERLET || (langevin && !c.stochastic_h && hyd);
@@ -146,8 +171,7 @@ __device__ __forceinline__ double md_atom(const PackView &v, const MDDev &d, con
       }
   } else if (langevin) {
     // md.cpp:1003-1040 with the step's constant quotients formed on the host
-    const double im = 1.0 / m;
-    double tim = t * im;
+    double tim = t * in.im;
     if (step > 0)
       for (int k = 0; k < 3; k++) vel[k] += c.kick1 * f[k] * tim;
     ke = 0.5 * m * (vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]);
@@ -161,9 +185,7 @@ __device__ __forceinline__ double md_atom(const PackView &v, const MDDev &d, con
         md_normals(v, d, step, i, nr);
       }
       double n1x = nr[0], n2y = nr[1], n2x = nr[2], n1z = nr[3], n1y = nr[4], n2z = nr[5];
-      double kTdivm = d.kB * c.temp * im;
-      double sigmav = sqrt(kTdivm * c.varv);
-      double sigmar = sqrt(kTdivm * c.varr) * c.inv_gamma;
+      const double sigmav = in.sigmav, sigmar = in.sigmar;
       double sq = c.sq_crv;
       double dvr[3] = {sigmav * (c.crv * n1x + sq * n2x), sigmav * (c.crv * n1y + sq * n2y),
                        sigmav * (c.crv * n1z + sq * n2z)};

@@ -279,11 +279,16 @@ void pdgpu_server::enqueue_min_chunk(Job *j) {
     int cnt = j->counter + j->iter + q;
     key += (p.UpdateNList > 0 && (cnt % p.UpdateNList) == 0) ? '1' : '0';
   }
+  const MinCtl ctl = min_ctl(e->min_state, p.Algorithm, slope, p.Strictness, steps);
   auto enqueue = [&]() {
     for (int q = 0; q < j->chunk; q++) {
-      if (key[key.size() - j->chunk + q] == '1') rebuild_pairs(P, j->st);
-      calc_forces_enqueue(j->st, e, true, min_step_src(e->min_state, false));
-      launch_min_step(P.v, j->st, e->min_state, p.Algorithm, slope, p.Strictness, p.StepSize, steps);
+      const bool rebuild = key[key.size() - j->chunk + q] == '1';
+      if (rebuild) rebuild_pairs(P, j->st);
+      EvalOpts o;
+      o.old_tiles = !rebuild && q > 0;
+      o.ctl = &ctl;
+      calc_forces_enqueue(j->st, e, true, min_step_src(e->min_state, false), o);
+      launch_min_update(P.v, j->st, ctl, p.StepSize);
     }
   };
   SysEntry::GraphSlot *g = nullptr;
