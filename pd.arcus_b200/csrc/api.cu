@@ -1374,11 +1374,62 @@ int pdgpu_sasa_lcpo_get(pdgpu_ctx *c, int32_t sys, double *sasa, double *deriv) 
 }
 }  // extern "C"
 
+// Does an MD step's energy record go to the pack's third stream?  Where the
+// steps alternate energy buffers: buffer b is written again by step q + 2,
+// after the integrator of q + 1 has waited for this record.  With the surface
+// term it stays on the second stream, whose next launch reads the step
+// counter that the record advances.
+static bool record_apart(const Pack &P) {
+  return P.rec && P.v.tile_mode && !P.slow() && P.v.lc.update <= 0;
+}
+static void launch_record(cudaStream_t st, SysEntry *e, int b) {
+  Pack &P = *e->pack;
+  const cudaStream_t rec = record_apart(P) ? P.rec : P.side;
+  cudaEventRecord(P.fork2, st);
+  cudaStreamWaitEvent(rec, P.fork2, 0);
+  PackView vb = P.v;
+  vb.ebuf = b;
+  launch_energy(vb, rec,
+                pair_energy_mode(P) | (has_bonded(P) ? EM_BONDED : 0) | (P.v.lc.update > 0 ? EM_SURF : 0) |
+                    EM_KINETIC | EM_RECORD | EM_ASSIGN,
+                e->hist, e->step_dev);
+  cudaEventRecord(P.ene_done[b], rec);
+  P.ene_pending[b] = true;
+}
+// The record that record_due holds back, if any.
+static void flush_record(cudaStream_t st, SysEntry *e) {
+  Pack &P = *e->pack;
+  if (P.record_due < 0) return;
+  const int b = P.record_due;
+  P.record_due = -1;
+  launch_record(st, e, b);
+}
+
 // Forcefield::calcForces for {FF_Bonded, GB[, FF_SASA_LCPO]}: the bonded
 // terms and the surface term (zeroing their accumulators first) run on the
 // pack's second stream beside the three pair passes; the stream joins
 // before the energies are read.  The surface term reads the step counter
 // after the previous step's energy record, which runs on that stream too.
+//
+// When they start beside the three launches of a tile evaluation: a small pack
+// is bound by phase A's chain of loads, which the warps of the bonded terms
+// and of the previous step's record lengthen on the SMs they share, and both
+// are shorter than B and C: they go behind A.  A large pack is bound by what
+// all the kernels issue, and what starts later ends later: at once.
+// kBehindA lies between the two; MD step, both kernels on one stream from
+// the start -> on two streams -> on two streams behind A:
+//   without rebuilds, 12 A: 133 atoms 21.0 -> 19.0 -> 18.4 us, 506 17.1 ->
+//   17.2 -> 15.1, 985 18.0 -> 18.7 -> 15.7, 1,662 20.8 -> 19.8 -> 17.5, 2,972
+//   21.9 -> 21.9 -> 19.5, 5,073 26.1 -> 23.6 -> 22.5
+//   rebuilds every 10 steps, 16 A: 5,073 atoms - -> 28.5 -> 30.2 us, 20,566 59.9 ->
+//   56.0 -> 57.9; 8 peptides, 12 A: - -> 48.4 -> 49.6, 64: 215 -> 203 -> 212
+// (The record behind B: 20.0 us at 985 atoms, it then ends after C.)  The surface
+// term is longer than B and C and starts at once, the bonded terms before
+// it; so does all with the cooperative launch or the row passes.
+static constexpr int kBehindA = 4096;
+static bool behind_first_phase(const Pack &P, bool coop) {
+  return P.v.tile_mode && P.v.n_atoms <= kBehindA && P.v.lc.update <= 0 && eval_tiles_split(P.v, coop);
+}
 void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce) {
   StepSrc step;
   step.imm = e->ws_step;
@@ -1390,14 +1441,21 @@ void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepS
   const bool bonded = has_bonded(P);
   const bool surf = P.v.lc.update > 0;
   const bool side = bonded || surf;
-  if (side) {
+  auto side_terms = [&] {
     cudaEventRecord(P.fork, st);
     cudaStreamWaitEvent(P.side, P.fork, 0);
     cudaMemsetAsync(P.v.fx, 0, sizeof(long long) * 3 * (size_t)P.v.n_atoms, P.side);  // fx, fy, fz: one block
-    if (bonded) launch_bonded_terms(P.v, P.side);
+    if (bonded) {
+      PackView vb = P.v;
+      vb.ebuf = ebuf;
+      launch_bonded_terms(vb, P.side);
+    }
     if (surf) launch_lcpo(P.v, P.side, step, false, P.csr_stale);
     cudaEventRecord(P.join, P.side);
-  }
+  };
+  const bool coop = o.coop < 0 ? P.coop : o.coop != 0;
+  const bool behind = behind_first_phase(P, coop);
+  if (side && !behind) side_terms();
   // with an MD step's energy record still running beside, the record is
   // left to it (it forms the record from zero) and the fused pass, which
   // writes what the record reads, waits for it
@@ -1413,7 +1471,14 @@ void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepS
     if (slow) P.wait_energy(st, ebuf ^ 1);
     PackView vb = P.v;
     vb.ebuf = ebuf;
-    launch_eval_tiles(vb, st, zero | (o.old_tiles ? ZF_OLD_TILES : 0), o.coop < 0 ? P.coop : o.coop != 0);
+    auto others = [&] {
+      if (side) side_terms();
+      flush_record(st, e);
+    };
+    BehindA ba;
+    ba.fn = [](void *f) { (*static_cast<decltype(others) *>(f))(); };
+    ba.ctx = &others;
+    launch_eval_tiles(vb, st, zero | (o.old_tiles ? ZF_OLD_TILES : 0), coop, behind ? ba : BehindA());
     P.last_ebuf = ebuf;
   } else {
     launch_born_radii(P.v, st, zero);
@@ -1565,18 +1630,11 @@ void pdgpu::md_step_enqueue(cudaStream_t st, SysEntry *e, const MDCoef &k, int q
   P.wait_energy(st, b);
   launch_md_step_impl(P.v, st, k, nullptr, e->step_dev, P.is_h, e->seeds, e->traj_dev, e->traj_every,
                       e->traj_dev_cap);
-  // the step's energy record on the second stream, beside the next step's
-  // evaluation (its bonded terms queue behind it on that stream)
-  cudaEventRecord(P.fork2, st);
-  cudaStreamWaitEvent(P.side, P.fork2, 0);
-  PackView vb = P.v;
-  vb.ebuf = b;
-  launch_energy(vb, P.side,
-                pair_energy_mode(P) | (has_bonded(P) ? EM_BONDED : 0) | (P.v.lc.update > 0 ? EM_SURF : 0) |
-                    EM_KINETIC | EM_RECORD | EM_ASSIGN,
-                e->hist, e->step_dev);
-  cudaEventRecord(P.ene_done[b], P.side);
-  P.ene_pending[b] = true;
+  // the step's energy record beside the next step's evaluation
+  if (record_apart(P) && behind_first_phase(P, P.coop_md))
+    P.record_due = b;
+  else
+    launch_record(st, e, b);
 }
 // Trajectory frames of steps [s0, s1) (absolute): mirrored from the device
 // ring into the host ring on the pack's second stream once the steps are
@@ -1613,6 +1671,7 @@ static void trajectory_copy(pdgpu_ctx *c, SysEntry *e, int s0, int s1) {
 // main stream.
 void pdgpu::md_steps_end(cudaStream_t st, SysEntry *e) {
   Pack &P = *e->pack;
+  flush_record(st, e);
   P.wait_energy(st, 0);
   P.wait_energy(st, 1);
 }
@@ -1728,6 +1787,7 @@ static int md_run_impl(pdgpu_ctx *c, SysEntry *e, const pdgpu_md_params *p, int3
     if (r) return r;
   }
   if ((r = ready_pairs(c, e))) return r;
+  if (!P.rec) PDGPU_CUDA(cudaStreamCreateWithFlags(&P.rec, cudaStreamNonBlocking));
   // A block is one list period: [rebuild] + UpdateNList steps.  If the
   // in-block rebuild overflows the list buffer, every kernel after it skips
   // (device flag), the state stays at the block start, and the host grows

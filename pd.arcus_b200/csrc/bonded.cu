@@ -185,17 +185,18 @@ __global__ void k_bonded_all(PackView v) {
   if (v.flags[F_NL_OVERFLOW]) return;  // the step is being re-planned
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   const BondedTerms &b = v.bt;
+  const int alt = v.ebuf ? 1 : 0;  // the energy buffer
   if (t < b.nb) {
-    bond_term(v, t, b.e_bond, b.vir_bond);
+    bond_term(v, t, b.e_bond + alt * (size_t)b.nb, b.vir_bond + alt * (size_t)b.nb);
     return;
   }
   t -= b.nb;
   if (t < b.na) {
-    angle_term(v, t, b.e_angle);
+    angle_term(v, t, b.e_angle + alt * (size_t)b.na);
     return;
   }
   t -= b.na;
-  if (t < b.nt + b.ni) dihedral_term(v, t, b.e_dih);
+  if (t < b.nt + b.ni) dihedral_term(v, t, b.e_dih + alt * (size_t)(b.nt + b.ni));
 }
 
 void launch_bonded_terms(const PackView &v, cudaStream_t st) {

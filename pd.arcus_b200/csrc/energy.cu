@@ -107,11 +107,14 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energy(PackView v, int mode,
   if (surf) sh[P_SURF][x] = chunk_sum(v.e_atom + (size_t)AE_SURF * N, lo[0], hi[0]);
   if (kin) sh[P_KIN][x] = chunk_sum(v.e_atom + (size_t)AE_KIN * N, lo[0], hi[0]);
   if (bonded) {
-    sh[P_BOND][x] = chunk_sum(v.bt.e_bond, lo[1], hi[1]);
-    sh[P_BVIR][x] = chunk_sum(v.bt.vir_bond, lo[1], hi[1]);
-    sh[P_ANGLE][x] = chunk_sum(v.bt.e_angle, lo[2], hi[2]);
+    const BondedTerms &t = v.bt;
+    const size_t alt = v.ebuf ? 1 : 0;
+    sh[P_BOND][x] = chunk_sum(t.e_bond + alt * t.nb, lo[1], hi[1]);
+    sh[P_BVIR][x] = chunk_sum(t.vir_bond + alt * t.nb, lo[1], hi[1]);
+    sh[P_ANGLE][x] = chunk_sum(t.e_angle + alt * t.na, lo[2], hi[2]);
     // torsions and impropers share the dihedral array: two ranges
-    sh[P_DIH][x] = chunk_sum(v.bt.e_dih, lo[3], hi[3]) + chunk_sum(v.bt.e_dih, lo[4], hi[4]);
+    const double *dih = t.e_dih + alt * (t.nt + t.ni);
+    sh[P_DIH][x] = chunk_sum(dih, lo[3], hi[3]) + chunk_sum(dih, lo[4], hi[4]);
   }
   if (overflow) return;
   __syncthreads();

@@ -1282,10 +1282,14 @@ static cudaError_t launch_ev(int ph, const PackView &v, cudaStream_t st, int zer
 
 // The three GB passes on the tiles: one cooperative launch when allowed,
 // else three launches of the same phases.
-cudaError_t launch_eval_tiles(const PackView &v, cudaStream_t st, int zero, bool coop) {
+bool eval_tiles_split(const PackView &v, bool coop) {
+  return v.n_sc && v.ev_blocks > 0 && !(coop && fused_wanted());
+}
+cudaError_t launch_eval_tiles(const PackView &v, cudaStream_t st, int zero, bool coop, BehindA behind_a) {
   if (!v.n_sc || v.ev_blocks <= 0) return cudaSuccess;
-  if (coop && fused_wanted()) return launch_ev(7, v, st, zero, true);
+  if (!eval_tiles_split(v, coop)) return launch_ev(7, v, st, zero, true);
   cudaError_t e = launch_ev(1, v, st, zero, false);
+  if (behind_a.fn) behind_a.fn(behind_a.ctx);
   if (e == cudaSuccess) e = launch_ev(2, v, st, 0, false);
   if (e == cudaSuccess) e = launch_ev(4, v, st, 0, false);
   return e;

@@ -138,6 +138,7 @@ struct MinCtl {
 struct BondedTerms {
   int nb = 0, na = 0, nt = 0, ni = 0;
   const int *term_off = nullptr;  // [4*(S+1)]: bond, angle, torsion, improper ranges per system
+  // per-term energies, two buffers each (of nb, na and nt + ni terms; PackView::ebuf picks one)
   double *e_bond = nullptr, *vir_bond = nullptr, *e_angle = nullptr, *e_dih = nullptr;
   int2 *bij = nullptr;        // bond atoms (global)
   double2 *blk = nullptr;     // (l, k kcal/mol/A^2)
@@ -236,8 +237,9 @@ struct PackView {
   int *sys_flags;             // [S] SysFlag bits of the current evaluation
   // energy buffer 1 (ebuf): the evaluation kernel on the tiles and the
   // energy record of an MD step alternate between two copies of the pair
-  // slots of e_atom (AE_VDW .. AE_POL_SELF) and of sys_flags, so a step's
-  // record can run beside the next step's evaluation
+  // slots of e_atom (AE_VDW .. AE_POL_SELF), of sys_flags and of the bonded
+  // terms' energies, so a step's record can run beside the next step's
+  // evaluation and bonded terms
   double *e_pair_alt;         // [4N]
   int *sys_flags_alt;         // [S]
   int ebuf;                   // 0: e_atom / sys_flags, 1: the copies (set per launch)
@@ -317,10 +319,13 @@ struct Pack {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // the bonded terms run on a second stream beside the pair passes
   cudaStream_t side = nullptr;
+  // and an MD step's energy record on a third (made by the first MD run), so
+  // the next step's bonded terms do not queue behind it
+  cudaStream_t rec = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
-  // an MD step's energy record runs on the second stream beside the next
-  // step's first passes; the next writer of what it reads waits on its
-  // ene_done event.  On the tile layout step q of a block records from
+  // an MD step's energy record runs beside the next step's passes; the next
+  // writer of what it reads waits on its ene_done event.  On the tile layout
+  // step q of a block records from
   // energy buffer q & 1 (PackView::ebuf): the evaluation of step q + 1
   // writes the other buffer and does not wait; the evaluation of step q + 2
   // and the integrator of step q + 1 (it writes the kinetic energies the
@@ -329,7 +334,11 @@ struct Pack {
   cudaEvent_t fork2 = nullptr, ene_done[2] = {nullptr, nullptr};
   bool ene_pending[2] = {false, false};
   int last_ebuf = 0;             // buffer of the last evaluation's per-atom energies
-  bool energy_pending() const { return ene_pending[0] || ene_pending[1]; }
+  // the last step's record is still to be launched, from this buffer (-1:
+  // none): on the third stream it goes behind the next step's first phase, or
+  // to the end of the steps (flush_record)
+  int record_due = -1;
+  bool energy_pending() const { return ene_pending[0] || ene_pending[1] || record_due >= 0; }
   // a member has FastMode off: the vacuum LJ/Coulomb come from the
   // stand-alone pass over the neighbour-list rows
   bool slow() const {
@@ -421,7 +430,14 @@ void launch_gb_chain_tile(const PackView &v, cudaStream_t st);
 // LJ + Coulomb, chain rule, with the finish steps folded in; one
 // cooperative launch when `coop` (and PDGPU_FUSED is not 0), else three
 // launches of the same phases.  zero: ZeroFlags, as launch_born_radii.
-cudaError_t launch_eval_tiles(const PackView &v, cudaStream_t st, int zero, bool coop);
+// With three launches behind_a is called between the first and the second:
+// what it puts on other streams starts when the first phase has ended.
+struct BehindA {
+  void (*fn)(void *) = nullptr;
+  void *ctx = nullptr;
+};
+cudaError_t launch_eval_tiles(const PackView &v, cudaStream_t st, int zero, bool coop, BehindA behind_a = {});
+bool eval_tiles_split(const PackView &v, bool coop);  // three launches?
 int eval_tiles_grid(long long tile_cap);
 // the three phases one launch each, timed with events on `st` (ms[0..2]),
 // then the single cooperative launch (ms[3])

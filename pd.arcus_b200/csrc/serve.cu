@@ -545,6 +545,10 @@ void pdgpu_server::admit(Job *j, const std::vector<Job *> &more) {
     cudaMemcpyAsync(P.v.oz, P.v.z, sizeof(double) * n, cudaMemcpyDeviceToDevice, j->st);
     enqueue_size(j, PH_MIN);
   } else if (j->spec.kind == PDGPU_JOB_MD) {
+    if (!P.rec && cudaStreamCreateWithFlags(&P.rec, cudaStreamNonBlocking) != cudaSuccess) {
+      P.rec = nullptr;  // the energy records share the bonded terms' stream
+      cudaGetLastError();
+    }
     // history [step][member][3]
     if (xalloc(e, &e->hist, (size_t)3 * j->spec.steps * S) != cudaSuccess) {
       fail(j, PDGPU_ERR_NOMEM, "device allocation failed (MD history)");

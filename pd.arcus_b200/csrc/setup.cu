@@ -223,6 +223,7 @@ Pack::~Pack() {
   for (auto &ev : ene_done)
     if (ev) cudaEventDestroy(ev);
   if (side) cudaStreamDestroy(side);
+  if (rec) cudaStreamDestroy(rec);
   if (cur >= 0 && cur != device) cudaSetDevice(cur);
 }
 
@@ -719,10 +720,11 @@ Pack *pack_create(int device, cudaStream_t st, const std::vector<const SystemHos
   PALLOC(toff_d, toff.size());
   cudaMemcpyAsync(toff_d, toff.data(), sizeof(int) * toff.size(), cudaMemcpyHostToDevice, st);
   bt.term_off = toff_d;
-  PALLOC(bt.e_bond, bt.nb);
-  PALLOC(bt.vir_bond, bt.nb);
-  PALLOC(bt.e_angle, bt.na);
-  PALLOC(bt.e_dih, ndih);
+  // (two energy buffers each, PackView::ebuf)
+  PALLOC(bt.e_bond, 2 * (size_t)bt.nb);
+  PALLOC(bt.vir_bond, 2 * (size_t)bt.nb);
+  PALLOC(bt.e_angle, 2 * (size_t)bt.na);
+  PALLOC(bt.e_dih, 2 * (size_t)ndih);
   // backbone torsion moves and hydrogen flags
   {
     std::vector<int2> rax;
