@@ -1382,11 +1382,10 @@ int pdgpu_sasa_lcpo_get(pdgpu_ctx *c, int32_t sys, double *sasa, double *deriv) 
 static bool record_apart(const Pack &P) {
   return P.rec && P.v.tile_mode && !P.slow() && P.v.lc.update <= 0;
 }
-static void launch_record(cudaStream_t st, SysEntry *e, int b) {
+static void launch_record(SysEntry *e, int b, cudaEvent_t after) {
   Pack &P = *e->pack;
   const cudaStream_t rec = record_apart(P) ? P.rec : P.side;
-  cudaEventRecord(P.fork2, st);
-  cudaStreamWaitEvent(rec, P.fork2, 0);
+  cudaStreamWaitEvent(rec, after, 0);
   PackView vb = P.v;
   vb.ebuf = b;
   launch_energy(vb, rec,
@@ -1397,12 +1396,12 @@ static void launch_record(cudaStream_t st, SysEntry *e, int b) {
   P.ene_pending[b] = true;
 }
 // The record that record_due holds back, if any.
-static void flush_record(cudaStream_t st, SysEntry *e) {
+static void flush_record(SysEntry *e, cudaEvent_t after) {
   Pack &P = *e->pack;
   if (P.record_due < 0) return;
   const int b = P.record_due;
   P.record_due = -1;
-  launch_record(st, e, b);
+  launch_record(e, b, after);
 }
 
 // Forcefield::calcForces for {FF_Bonded, GB[, FF_SASA_LCPO]}: the bonded
@@ -1442,9 +1441,7 @@ void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepS
   const bool surf = P.v.lc.update > 0;
   const bool side = bonded || surf;
   auto side_terms = [&] {
-    cudaEventRecord(P.fork, st);
     cudaStreamWaitEvent(P.side, P.fork, 0);
-    cudaMemsetAsync(P.v.fx, 0, sizeof(long long) * 3 * (size_t)P.v.n_atoms, P.side);  // fx, fy, fz: one block
     if (bonded) {
       PackView vb = P.v;
       vb.ebuf = ebuf;
@@ -1455,12 +1452,18 @@ void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepS
   };
   const bool coop = o.coop < 0 ? P.coop : o.coop != 0;
   const bool behind = behind_first_phase(P, coop);
-  if (side && !behind) side_terms();
+  const bool first = side && !behind;
+  if (first) {
+    cudaEventRecord(P.fork, st);
+    cudaStreamWaitEvent(P.side, P.fork, 0);
+    cudaMemsetAsync(P.v.fx, 0, sizeof(long long) * 3 * (size_t)P.v.n_atoms, P.side);  // fx, fy, fz: one block
+    side_terms();
+  }
   // with an MD step's energy record still running beside, the record is
   // left to it (it forms the record from zero) and the fused pass, which
   // writes what the record reads, waits for it
   const bool pending = P.energy_pending();
-  const int zero = ZF_PAIRS | (side ? 0 : ZF_BONDED) | (pending ? 0 : ZF_RECORD);
+  const int zero = ZF_PAIRS | (first ? 0 : ZF_BONDED) | (pending ? 0 : ZF_RECORD);
   const bool slow = P.slow();
   if (P.v.tile_mode) {
     // the tile layout: the three passes as one evaluation into energy
@@ -1471,14 +1474,11 @@ void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepS
     if (slow) P.wait_energy(st, ebuf ^ 1);
     PackView vb = P.v;
     vb.ebuf = ebuf;
-    auto others = [&] {
+    launch_eval_tiles(vb, st, zero | (o.old_tiles ? ZF_OLD_TILES : 0), coop, behind ? P.fork : nullptr);
+    if (behind) {  // after the three launches, which the device waits for
       if (side) side_terms();
-      flush_record(st, e);
-    };
-    BehindA ba;
-    ba.fn = [](void *f) { (*static_cast<decltype(others) *>(f))(); };
-    ba.ctx = &others;
-    launch_eval_tiles(vb, st, zero | (o.old_tiles ? ZF_OLD_TILES : 0), coop, behind ? ba : BehindA());
+      flush_record(e, P.fork);
+    }
     P.last_ebuf = ebuf;
   } else {
     launch_born_radii(P.v, st, zero);
@@ -1631,10 +1631,12 @@ void pdgpu::md_step_enqueue(cudaStream_t st, SysEntry *e, const MDCoef &k, int q
   launch_md_step_impl(P.v, st, k, nullptr, e->step_dev, P.is_h, e->seeds, e->traj_dev, e->traj_every,
                       e->traj_dev_cap);
   // the step's energy record beside the next step's evaluation
-  if (record_apart(P) && behind_first_phase(P, P.coop_md))
+  if (record_apart(P) && behind_first_phase(P, P.coop_md)) {
     P.record_due = b;
-  else
-    launch_record(st, e, b);
+  } else {
+    cudaEventRecord(P.fork2, st);
+    launch_record(e, b, P.fork2);
+  }
 }
 // Trajectory frames of steps [s0, s1) (absolute): mirrored from the device
 // ring into the host ring on the pack's second stream once the steps are
@@ -1671,7 +1673,10 @@ static void trajectory_copy(pdgpu_ctx *c, SysEntry *e, int s0, int s1) {
 // main stream.
 void pdgpu::md_steps_end(cudaStream_t st, SysEntry *e) {
   Pack &P = *e->pack;
-  flush_record(st, e);
+  if (P.record_due >= 0) {
+    cudaEventRecord(P.fork2, st);
+    flush_record(e, P.fork2);
+  }
   P.wait_energy(st, 0);
   P.wait_energy(st, 1);
 }

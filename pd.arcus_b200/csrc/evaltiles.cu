@@ -1285,11 +1285,11 @@ static cudaError_t launch_ev(int ph, const PackView &v, cudaStream_t st, int zer
 bool eval_tiles_split(const PackView &v, bool coop) {
   return v.n_sc && v.ev_blocks > 0 && !(coop && fused_wanted());
 }
-cudaError_t launch_eval_tiles(const PackView &v, cudaStream_t st, int zero, bool coop, BehindA behind_a) {
+cudaError_t launch_eval_tiles(const PackView &v, cudaStream_t st, int zero, bool coop, cudaEvent_t behind_a) {
   if (!v.n_sc || v.ev_blocks <= 0) return cudaSuccess;
   if (!eval_tiles_split(v, coop)) return launch_ev(7, v, st, zero, true);
   cudaError_t e = launch_ev(1, v, st, zero, false);
-  if (behind_a.fn) behind_a.fn(behind_a.ctx);
+  if (behind_a) cudaEventRecord(behind_a, st);
   if (e == cudaSuccess) e = launch_ev(2, v, st, 0, false);
   if (e == cudaSuccess) e = launch_ev(4, v, st, 0, false);
   return e;

@@ -430,13 +430,10 @@ void launch_gb_chain_tile(const PackView &v, cudaStream_t st);
 // LJ + Coulomb, chain rule, with the finish steps folded in; one
 // cooperative launch when `coop` (and PDGPU_FUSED is not 0), else three
 // launches of the same phases.  zero: ZeroFlags, as launch_born_radii.
-// With three launches behind_a is called between the first and the second:
-// what it puts on other streams starts when the first phase has ended.
-struct BehindA {
-  void (*fn)(void *) = nullptr;
-  void *ctx = nullptr;
-};
-cudaError_t launch_eval_tiles(const PackView &v, cudaStream_t st, int zero, bool coop, BehindA behind_a = {});
+// With three launches the event behind_a is recorded between the first and
+// the second: what waits for it starts when the first phase has ended.
+cudaError_t launch_eval_tiles(const PackView &v, cudaStream_t st, int zero, bool coop,
+                              cudaEvent_t behind_a = nullptr);
 bool eval_tiles_split(const PackView &v, bool coop);  // three launches?
 int eval_tiles_grid(long long tile_cap);
 // the three phases one launch each, timed with events on `st` (ms[0..2]),
