@@ -1382,7 +1382,7 @@ int pdgpu_sasa_lcpo_get(pdgpu_ctx *c, int32_t sys, double *sasa, double *deriv) 
 static bool record_apart(const Pack &P) {
   return P.rec && P.v.tile_mode && !P.slow() && P.v.lc.update <= 0;
 }
-static void launch_record(SysEntry *e, int b, cudaEvent_t after) {
+static void launch_record(SysEntry *e, int b, bool gate, cudaEvent_t after) {
   Pack &P = *e->pack;
   const cudaStream_t rec = record_apart(P) ? P.rec : P.side;
   cudaStreamWaitEvent(rec, after, 0);
@@ -1390,7 +1390,7 @@ static void launch_record(SysEntry *e, int b, cudaEvent_t after) {
   vb.ebuf = b;
   launch_energy(vb, rec,
                 pair_energy_mode(P) | (has_bonded(P) ? EM_BONDED : 0) | (P.v.lc.update > 0 ? EM_SURF : 0) |
-                    EM_KINETIC | EM_RECORD | EM_ASSIGN,
+                    EM_KINETIC | EM_RECORD | EM_ASSIGN | (gate ? EM_GATE : 0),
                 e->hist, e->step_dev);
   cudaEventRecord(P.ene_done[b], rec);
   P.ene_pending[b] = true;
@@ -1401,7 +1401,7 @@ static void flush_record(SysEntry *e, cudaEvent_t after) {
   if (P.record_due < 0) return;
   const int b = P.record_due;
   P.record_due = -1;
-  launch_record(e, b, after);
+  launch_record(e, b, P.gate_due, after);
 }
 
 // Forcefield::calcForces for {FF_Bonded, GB[, FF_SASA_LCPO]}: the bonded
@@ -1614,7 +1614,7 @@ int pdgpu_md_init_velocities(pdgpu_ctx *c, int32_t sys, double temperature, uint
 // one MD step enqueue: forces, integrate, one energy reduction that also
 // records the step and advances the device step counter (7 launches)
 }  // extern "C"
-void pdgpu::md_step_enqueue(cudaStream_t st, SysEntry *e, const MDCoef &k, int q) {
+void pdgpu::md_step_enqueue(cudaStream_t st, SysEntry *e, const MDCoef &k, int q, bool gate) {
   Pack &P = *e->pack;
   StepSrc step;
   step.p = e->step_dev;  // MolecularDynamics::run_core sets WorkSpace::Step = Step (md.cpp:214)
@@ -1633,9 +1633,10 @@ void pdgpu::md_step_enqueue(cudaStream_t st, SysEntry *e, const MDCoef &k, int q
   // the step's energy record beside the next step's evaluation
   if (record_apart(P) && behind_first_phase(P, P.coop_md)) {
     P.record_due = b;
+    P.gate_due = gate;
   } else {
     cudaEventRecord(P.fork2, st);
-    launch_record(e, b, P.fork2);
+    launch_record(e, b, gate, P.fork2);
   }
 }
 // Trajectory frames of steps [s0, s1) (absolute): mirrored from the device
@@ -1797,135 +1798,182 @@ static int md_run_impl(pdgpu_ctx *c, SysEntry *e, const pdgpu_md_params *p, int3
   // in-block rebuild overflows the list buffer, every kernel after it skips
   // (device flag), the state stays at the block start, and the host grows
   // the buffer and runs the block again.
-  if (!e->pin_flags && cudaHostAlloc((void **)&e->pin_flags, sizeof(int) * (F_COUNT + 3), 0) != cudaSuccess) {
+  //
+  // The host reads a block's flags while the next block runs (the wake-up and
+  // the launch between two: step of a 10-step period 17.1 -> 16.5 us at 133
+  // atoms, 19.0 -> 18.5 at 985, 20.9 -> 20.2 at 1,662, 55.4 -> 54.6 at 20,566).
+  // A block enqueued behind one that failed does nothing: an overflow's flag is
+  // still set, and after a NaN or a full overlap list the last record sets it
+  // (EM_GATE), so the state is the failed block's.  Not with trajectory
+  // frames (each block's are copied before the next writes the ring) nor with the
+  // cooperative launch (its barrier's counters are mended between blocks).
+  if (!e->pin_flags && cudaHostAlloc((void **)&e->pin_flags, sizeof(int) * (2 * F_COUNT + 3), 0) != cudaSuccess) {
     e->pin_flags = nullptr;
     set_error("page-locked host allocation failed (MD flags)");
     return PDGPU_ERR_NOMEM;
   }
-  int *steps0 = e->pin_flags + F_COUNT;  // step counter, first step, finished-system count
+  for (cudaEvent_t &ev : e->block_ev)
+    if (!ev) PDGPU_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  int *steps0 = e->pin_flags + 2 * F_COUNT;  // step counter, first step, finished-system count
   steps0[0] = steps0[1] = first_step;
   steps0[2] = 0;
   PDGPU_CUDA(cudaMemcpyAsync(e->step_dev, steps0, sizeof(int) * 3, cudaMemcpyHostToDevice, c->st));
   cudaEventRecord(P.ev0, c->st);
-  int s = 0;
-  while (s < steps) {
-    int step = first_step + s;
+  // One block of the run's steps from s, enqueued with its flag copy.
+  struct Block {
+    int s, n, slot;
+  };
+  auto enqueue_block = [&](int s, int counter, Block *out) -> int {
     // Blocks follow the list periods (protocolbase.cpp:113-122: a rebuild
     // when the step counter is a multiple of UpdateNList).  A run that
     // starts inside a period first finishes that period in one block
     // without a rebuild; a run that ends inside one ends with a shorter
     // block that begins with the rebuild.  Every block of more than one
     // step replays a cached graph of its own shape.
-    bool rebuild = every > 0 && (P.nlist_counter % every) == 0;
+    const bool rebuild = every > 0 && (counter % every) == 0;
     int block = 1;
     if (every > 1) {
-      const int left = rebuild ? every : every - P.nlist_counter % every;
+      const int left = rebuild ? every : every - counter % every;
       block = std::min(left, steps - s);
     }
-    bool use_graph = p->UseGraph && block > 1;
-    int counter0 = P.nlist_counter;
-    for (int attempt = 0;; attempt++) {
-      if (attempt == 4) {
+    auto enqueue = [&] {
+      if (rebuild) rebuild_enqueue(P, c->st);
+      for (int q = 0; q < block; q++) md_step_enqueue(c->st, e, k, q, q == block - 1);
+      md_steps_end(c->st, e);
+    };
+    const bool use_graph = p->UseGraph && block > 1;
+    for (bool again = true; again;) {
+      again = false;
+      if (!use_graph) {
+        enqueue();
+        break;
+      }
+      // graphs are cached per system; the key holds every value baked in
+      char key[288];
+      snprintf(key, sizeof key, "%d|%d|%p|%lld|%p|%d|%d|%.17g|%.17g|%.17g|%d|%d|%d|%d%d%d|%d%d%d|%p|%d|%d", block,
+               (int)rebuild, (void *)v.nl, v.nl_cap, (void *)e->hist, k.integrator, k.steps, k.dt, k.gamma,
+               k.temp, k.stochastic_h, P.radix_passes, (int)e->host->params.FastMode, v.lpa[0], v.lpa[1],
+               v.lpa[2], v.tile_mode, (int)tile_search_ok(P), (int)P.coop_md, (void *)e->traj_dev, e->traj_every,
+               e->traj_dev_cap);
+      SysEntry::GraphSlot *g = nullptr;
+      for (auto &q : e->gslots)
+        if (q.key == key) g = &q;
+      if (!g) {
+        if ((int)e->gslots.size() >= SysEntry::kGraphSlots) {  // evict the least recently used
+          auto lru = std::min_element(e->gslots.begin(), e->gslots.end(),
+                                      [](const SysEntry::GraphSlot &a, const SysEntry::GraphSlot &b) {
+                                        return a.used < b.used;
+                                      });
+          if (int rs = sync_check(c, "md block")) return rs;  // it may be running
+          e->drop_slot(*lru);
+          e->gslots.erase(lru);
+        }
+        SysEntry::GraphSlot ng;
+        const bool pend0 = P.ene_pending[0], pend1 = P.ene_pending[1];  // both false between blocks
+        begin_capture_count();
+        PDGPU_CUDA(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
+        enqueue();
+        cudaError_t ce = cudaStreamEndCapture(c->st, &ng.graph);
+        ng.nodes = end_capture_count();
+        if (ce == cudaSuccess) ce = cudaGraphInstantiate(&ng.exec, ng.graph, 0);
+        if (ce != cudaSuccess) {
+          e->drop_slot(ng);
+          P.ene_pending[0] = pend0;
+          P.ene_pending[1] = pend1;
+          if (P.coop_md && P.v.tile_mode) {
+            // a graph that cannot hold the cooperative evaluation: the
+            // same phases as three launches from here on
+            cudaGetLastError();
+            P.coop_md = false;
+            again = true;
+            continue;
+          }
+          return cuda_fail(ce, "capture md block");
+        }
+        ng.key = key;
+        e->gslots.push_back(ng);
+        g = &e->gslots.back();
+      }
+      g->used = ++e->gclock;
+      PDGPU_CUDA(cudaGraphLaunch(g->exec, c->st));
+      launch_counter() += g->nodes;
+      e->graph_replays++;
+      if (rebuild) P.csr_stale = tile_search_ok(P);  // what the graph's rebuild made
+    }
+    if (s + block >= steps) cudaEventRecord(P.ev1, c->st);
+    PDGPU_CUDA(cudaMemcpyAsync(e->pin_flags + out->slot * F_COUNT, v.flags, sizeof(int) * F_COUNT,
+                               cudaMemcpyDeviceToHost, c->st));
+    PDGPU_CUDA(cudaEventRecord(e->block_ev[out->slot], c->st));
+    out->s = s;
+    out->n = block;
+    return PDGPU_OK;
+  };
+  const int counter0 = P.nlist_counter;
+  int done = 0, enqueued = 0, nrun = 0, attempt = 0, slot = 0;  // steps done and enqueued, blocks in flight
+  Block run[2];                                                 // oldest first
+  while (done < steps) {
+    while (nrun < (e->traj_every <= 0 && !P.coop_md ? 2 : 1) && enqueued < steps) {
+      run[nrun].slot = slot ^= 1;
+      if ((r = enqueue_block(enqueued, counter0 + enqueued, &run[nrun]))) {
+        cudaStreamSynchronize(c->st);
+        return r;
+      }
+      enqueued += run[nrun++].n;
+    }
+    const Block cur = run[0];
+    const bool last = cur.s + cur.n >= steps;
+    if (last && tail && (r = tail())) return r;
+    if (last) {
+      r = sync_check(c, "md block");
+    } else {
+      cudaError_t ce = cudaEventSynchronize(e->block_ev[cur.slot]);
+      if (ce == cudaSuccess) ce = cudaGetLastError();
+      r = ce == cudaSuccess ? PDGPU_OK : cuda_fail(ce, "md block");
+    }
+    if (r) return r;
+    const int *flags = e->pin_flags + cur.slot * F_COUNT;
+    if ((r = barrier_check(c, P, flags))) return r;
+    const bool cand = flags[F_LCPO_CAND], nan = flags[F_NAN], overflow = flags[F_NL_OVERFLOW] == 1;
+    if (cand || nan || overflow) {
+      // the block behind it has done nothing
+      if ((r = sync_check(c, "md block"))) return r;
+      if (cand || (nan && !overflow))  // the gate opens again
+        PDGPU_CUDA(cudaMemsetAsync(v.flags + F_NL_OVERFLOW, 0, sizeof(int), c->st));
+    }
+    if (cand) {
+      set_error(kLcpoCandMsg);
+      return PDGPU_ERR_STATE;
+    }
+    if (overflow) {
+      // state untouched since the block start: grow the list and re-run
+      if ((r = nlist_enqueue(c, e))) return r;
+      e->drop_graph();
+      if (++attempt == 4) {
         set_error("neighbour list kept overflowing after regrowth");
         return PDGPU_ERR_STATE;
       }
-      if (s > 0 || attempt > 0) {  // the first block starts from the run's own setup
-        PDGPU_CUDA(cudaMemsetAsync(v.flags + F_NL_OVERFLOW, 0, sizeof(int), c->st));
-        steps0[0] = step;
-        PDGPU_CUDA(cudaMemcpyAsync(e->step_dev, steps0, sizeof(int), cudaMemcpyHostToDevice, c->st));
-      }
-      if (use_graph) {
-        // graphs are cached per system; the key holds every value baked in
-        char key[288];
-        snprintf(key, sizeof key, "%d|%d|%p|%lld|%p|%d|%d|%.17g|%.17g|%.17g|%d|%d|%d|%d%d%d|%d%d%d|%p|%d|%d", block,
-                 (int)rebuild, (void *)v.nl, v.nl_cap, (void *)e->hist, k.integrator, k.steps, k.dt, k.gamma,
-                 k.temp, k.stochastic_h, P.radix_passes, (int)e->host->params.FastMode, v.lpa[0], v.lpa[1],
-                 v.lpa[2], v.tile_mode, (int)tile_search_ok(P), (int)P.coop_md, (void *)e->traj_dev, e->traj_every,
-                 e->traj_dev_cap);
-        SysEntry::GraphSlot *g = nullptr;
-        for (auto &q : e->gslots)
-          if (q.key == key) g = &q;
-        if (!g) {
-          if ((int)e->gslots.size() >= SysEntry::kGraphSlots) {  // evict the least recently used
-            auto lru = std::min_element(e->gslots.begin(), e->gslots.end(),
-                                        [](const SysEntry::GraphSlot &a, const SysEntry::GraphSlot &b) {
-                                          return a.used < b.used;
-                                        });
-            e->drop_slot(*lru);
-            e->gslots.erase(lru);
-          }
-          SysEntry::GraphSlot ng;
-          const bool pend0 = P.ene_pending[0], pend1 = P.ene_pending[1];  // both false between blocks
-          begin_capture_count();
-          PDGPU_CUDA(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-          if (rebuild) rebuild_enqueue(P, c->st);
-          for (int q = 0; q < block; q++) md_step_enqueue(c->st, e, k, q);
-          md_steps_end(c->st, e);
-          cudaError_t ce = cudaStreamEndCapture(c->st, &ng.graph);
-          ng.nodes = end_capture_count();
-          if (ce == cudaSuccess) ce = cudaGraphInstantiate(&ng.exec, ng.graph, 0);
-          if (ce != cudaSuccess) {
-            e->drop_slot(ng);
-            P.ene_pending[0] = pend0;
-            P.ene_pending[1] = pend1;
-            if (P.coop_md && P.v.tile_mode) {
-              // a graph that cannot hold the cooperative evaluation: the
-              // same phases as three launches from here on
-              cudaGetLastError();
-              P.coop_md = false;
-              continue;
-            }
-            return cuda_fail(ce, "capture md block");
-          }
-          ng.key = key;
-          e->gslots.push_back(ng);
-          g = &e->gslots.back();
-        }
-        g->used = ++e->gclock;
-        PDGPU_CUDA(cudaGraphLaunch(g->exec, c->st));
-        launch_counter() += g->nodes;
-        e->graph_replays++;
-        if (rebuild) P.csr_stale = tile_search_ok(P);  // what the graph's rebuild made
-      } else {
-        if (rebuild) rebuild_enqueue(P, c->st);
-        for (int q = 0; q < block; q++) md_step_enqueue(c->st, e, k, q);
-        md_steps_end(c->st, e);
-      }
-      const bool last = s + block >= steps;
-      if (last) {
-        cudaEventRecord(P.ev1, c->st);
-        if (tail && (r = tail())) return r;
-      }
-      int *flags = e->pin_flags;
-      PDGPU_CUDA(cudaMemcpyAsync(flags, v.flags, sizeof(int) * F_COUNT, cudaMemcpyDeviceToHost, c->st));
-      r = sync_check(c, "md block");
-      if (r) return r;
-      if ((r = barrier_check(c, P, flags))) return r;
-      if (flags[F_LCPO_CAND]) {
-        set_error(kLcpoCandMsg);
-        return PDGPU_ERR_STATE;
-      }
-      if (flags[F_NL_OVERFLOW]) {
-        // state untouched since the block start: grow the list and re-run
-        r = nlist_enqueue(c, e);
-        if (r) return r;
-        e->drop_graph();
-        continue;
-      }
-      if (flags[F_NAN]) {
-        if (history) {
-          std::vector<double> h((size_t)3 * (s + block) * S);
-          cudaMemcpy(h.data(), e->hist, sizeof(double) * h.size(), cudaMemcpyDeviceToHost);
-          for (size_t q = 0; q < h.size(); q++) history[q] = h[q] * consts().J_per_kcalmol;
-        }
-        set_error("Simulation unstable or division by zero (NaN energy)");
-        return PDGPU_ERR_UNSTABLE;
-      }
-      break;
+      PDGPU_CUDA(cudaMemsetAsync(v.flags + F_NL_OVERFLOW, 0, sizeof(int), c->st));
+      steps0[0] = first_step + done;
+      PDGPU_CUDA(cudaMemcpyAsync(e->step_dev, steps0, sizeof(int), cudaMemcpyHostToDevice, c->st));
+      enqueued = done;
+      nrun = 0;
+      continue;
     }
-    P.nlist_counter = counter0 + block;
-    trajectory_copy(c, e, step, step + block);
-    s += block;
+    if (nan) {
+      if (history) {
+        std::vector<double> h((size_t)3 * (done + cur.n) * S);
+        cudaMemcpy(h.data(), e->hist, sizeof(double) * h.size(), cudaMemcpyDeviceToHost);
+        for (size_t q = 0; q < h.size(); q++) history[q] = h[q] * consts().J_per_kcalmol;
+      }
+      set_error("Simulation unstable or division by zero (NaN energy)");
+      return PDGPU_ERR_UNSTABLE;
+    }
+    attempt = 0;
+    done += cur.n;
+    run[0] = run[1];
+    nrun--;
+    P.nlist_counter = counter0 + done;
+    trajectory_copy(c, e, first_step + cur.s, first_step + cur.s + cur.n);
   }
   if (e->traj_every > 0 && (r = sync_check(c, "md_run"))) return r;
   if (steps > 0) e->ws_step = first_step + steps - 1;  // WorkSpace::Step as run_core leaves it

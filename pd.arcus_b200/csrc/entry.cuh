@@ -89,9 +89,10 @@ struct SysEntry {
   void *min_state = nullptr;
   void *mc_state = nullptr;
   std::vector<void *> extra;
-  // page-locked: an MD run's flag read-back and step-counter upload
-  // ([F_COUNT] flags, then 3 ints); pdgpu_md_run_io's energies
+  // page-locked: an MD run's flag read-back (two blocks of [F_COUNT]) and
+  // step-counter upload (3 ints); pdgpu_md_run_io's energies
   int *pin_flags = nullptr;
+  cudaEvent_t block_ev[2] = {nullptr, nullptr};  // a block's flags are in pin_flags
   double *pin_ene = nullptr;
   double *io_stage = nullptr;  // [6N] device staging of pdgpu_md_run_io's state (an `extra` allocation)
   // cached MD block graph (the request loop's job graph)
@@ -135,6 +136,10 @@ struct SysEntry {
     free_trajectory();
     if (pin_flags || pin_ene) cudaStreamSynchronize(st);  // no copy in flight into them
     if (pin_flags) cudaFreeHost(pin_flags);
+    for (cudaEvent_t &ev : block_ev) {
+      if (ev) cudaEventDestroy(ev);
+      ev = nullptr;
+    }
     if (pin_ene) cudaFreeHost(pin_ene);
     pin_flags = nullptr;
     pin_ene = nullptr;
@@ -185,7 +190,8 @@ struct EvalOpts {
 void calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepSrc step, const EvalOpts &o = EvalOpts());
 // one MD step: forces, integrator, energy record (+ step counter advance);
 // q = the step's index in its block (its energy buffer is q & 1 on tiles)
-void md_step_enqueue(cudaStream_t st, SysEntry *e, const MDCoef &k, int q);
+// (gate: EM_GATE for the record)
+void md_step_enqueue(cudaStream_t st, SysEntry *e, const MDCoef &k, int q, bool gate = false);
 void md_steps_end(cudaStream_t st, SysEntry *e);
 MDCoef md_coef(const pdgpu_md_params *p, int step, int steps);
 // grow a pack's list buffer to hold `total` entries (stream-ordered)

@@ -90,6 +90,7 @@ enum EnergyMode {
   EM_BONDED = 8,       // bond, angle, torsion, bond virial
   EM_KINETIC = 16,     // ekin, etot
   EM_RECORD = 32,      // history row + step counter advance (step loops)
+  EM_GATE = 512,       // with EM_RECORD: F_NL_OVERFLOW = 2 after a NaN or F_LCPO_CAND (the next block skips)
   EM_ASSIGN = 64,      // form the record from zero (its slots were not zeroed before the step)
   EM_SURF = 128,       // LCPO surface term: epot_surf
   EM_PAIR_GB_SLOW = 256  // GB with FastMode off (calcBornForces): pol + self added to epot alone;
@@ -338,6 +339,7 @@ struct Pack {
   // none): on the third stream it goes behind the next step's first phase, or
   // to the end of the steps (flush_record)
   int record_due = -1;
+  bool gate_due = false;  // that record's EM_GATE
   bool energy_pending() const { return ene_pending[0] || ene_pending[1] || record_due >= 0; }
   // a member has FastMode off: the vacuum LJ/Coulomb come from the
   // stand-alone pass over the neighbour-list rows
