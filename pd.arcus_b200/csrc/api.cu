@@ -1405,7 +1405,7 @@ static void flush_record(SysEntry *e, cudaEvent_t after) {
 }
 
 // Forcefield::calcForces for {FF_Bonded, GB[, FF_SASA_LCPO]}: the bonded
-// terms and the surface term (zeroing their accumulators first) run on the
+// terms or the surface term (zeroing the accumulators first) run on the
 // pack's second stream beside the three pair passes; the stream joins
 // before the energies are read.  The surface term reads the step counter
 // after the previous step's energy record, which runs on that stream too.
@@ -1422,9 +1422,12 @@ static void flush_record(SysEntry *e, cudaEvent_t after) {
 //   21.9 -> 21.9 -> 19.5, 5,073 26.1 -> 23.6 -> 22.5
 //   rebuilds every 10 steps, 16 A: 5,073 atoms - -> 28.5 -> 30.2 us, 20,566 59.9 ->
 //   56.0 -> 57.9; 8 peptides, 12 A: - -> 48.4 -> 49.6, 64: 215 -> 203 -> 212
-// (The record behind B: 20.0 us at 985 atoms, it then ends after C.)  The surface
-// term is longer than B and C and starts at once, the bonded terms before
-// it; so does all with the cooperative launch or the row passes.
+// (The record behind B: 20.0 us at 985 atoms, it then ends after C.)  With the
+// cooperative launch or the row passes all starts at once.  So does the
+// surface term, the longest of the chains (50 us at 5,073 atoms where the three
+// passes take 27), and the bonded terms then follow the passes: in front
+// of the surface term they delayed it (forces with the surface term 88 -> 77 us
+// at 5,073 atoms, an MD step 44.5 -> 39.6, with dependent launches of its kernels).
 static constexpr int kBehindA = 4096;
 static bool behind_first_phase(const Pack &P, bool coop) {
   return P.v.tile_mode && P.v.n_atoms <= kBehindA && P.v.lc.update <= 0 && eval_tiles_split(P.v, coop);
@@ -1439,25 +1442,22 @@ void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepS
   const int ebuf = o.ebuf;
   const bool bonded = has_bonded(P);
   const bool surf = P.v.lc.update > 0;
-  const bool side = bonded || surf;
-  auto side_terms = [&] {
-    cudaStreamWaitEvent(P.side, P.fork, 0);
-    if (bonded) {
-      PackView vb = P.v;
-      vb.ebuf = ebuf;
-      launch_bonded_terms(vb, P.side);
-    }
-    if (surf) launch_lcpo(P.v, P.side, step, false, P.csr_stale);
-    cudaEventRecord(P.join, P.side);
-  };
   const bool coop = o.coop < 0 ? P.coop : o.coop != 0;
   const bool behind = behind_first_phase(P, coop);
-  const bool first = side && !behind;
+  const bool side = bonded || surf, first = side && !behind;
+  PackView vb = P.v;
+  vb.ebuf = ebuf;
   if (first) {
     cudaEventRecord(P.fork, st);
     cudaStreamWaitEvent(P.side, P.fork, 0);
     cudaMemsetAsync(P.v.fx, 0, sizeof(long long) * 3 * (size_t)P.v.n_atoms, P.side);  // fx, fy, fz: one block
-    side_terms();
+    if (surf) {
+      if (bonded) cudaEventRecord(P.fork2, P.side);
+      launch_lcpo(P.v, P.side, step, false, P.csr_stale);
+    } else {
+      launch_bonded_terms(vb, P.side);
+    }
+    cudaEventRecord(P.join, P.side);
   }
   // with an MD step's energy record still running beside, the record is
   // left to it (it forms the record from zero) and the fused pass, which
@@ -1472,11 +1472,13 @@ void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepS
     // buffer 0)
     P.wait_energy(st, ebuf);
     if (slow) P.wait_energy(st, ebuf ^ 1);
-    PackView vb = P.v;
-    vb.ebuf = ebuf;
     launch_eval_tiles(vb, st, zero | (o.old_tiles ? ZF_OLD_TILES : 0), coop, behind ? P.fork : nullptr);
     if (behind) {  // after the three launches, which the device waits for
-      if (side) side_terms();
+      if (side) {
+        cudaStreamWaitEvent(P.side, P.fork, 0);
+        launch_bonded_terms(vb, P.side);
+        cudaEventRecord(P.join, P.side);
+      }
       flush_record(e, P.fork);
     }
     P.last_ebuf = ebuf;
@@ -1490,6 +1492,10 @@ void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepS
   }
   // FastMode off: FF_NonBonded::calcForces beside calcBornForces
   if (slow) launch_nonbonded(P.v, st, P.sp[0].elec_mode);
+  if (bonded && surf) {
+    cudaStreamWaitEvent(st, P.fork2, 0);
+    launch_bonded_terms(vb, st);
+  }
   if (side) cudaStreamWaitEvent(st, P.join, 0);
   if (o.ctl) launch_min_dots(P.v, st, *o.ctl);
   if (reduce)

@@ -58,6 +58,7 @@ __device__ __forceinline__ bool lcpo_overlaps(double d2, double rs) {
 // different atoms' counters instead of all to the same 32.
 template <bool EO>
 __global__ void __launch_bounds__(128) k_lcpo_cand_tiles(PackView v, StepSrc ss) {
+  PDGPU_DEP_ENTRY();
   if (v.flags[F_NL_OVERFLOW]) return;
   const LcpoView &lc = v.lc;
   const int lane = threadIdx.x & 31;
@@ -92,6 +93,7 @@ __global__ void __launch_bounds__(128) k_lcpo_cand_tiles(PackView v, StepSrc ss)
 
 template <bool EO, bool TILES>
 __global__ void __launch_bounds__(kLcpoWarps * 32) k_lcpo_list(PackView v, StepSrc ss) {
+  PDGPU_DEP_ENTRY();
   __shared__ int cand[kLcpoWarps][kLcpoCand];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const LcpoView &lc = v.lc;
@@ -177,6 +179,7 @@ __device__ __forceinline__ void lcpo_add_force(const PackView &v, int i, double 
 // different banks
 template <bool EO>
 __global__ void __launch_bounds__(kLcpoWarps * 32) k_lcpo_eval(PackView v, StepSrc ss) {
+  PDGPU_DEP_ENTRY();
   __shared__ double T[kLcpoWarps][kLcpoQ][kLcpoMax + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const LcpoView &lc = v.lc;
@@ -369,26 +372,26 @@ void launch_lcpo_part(const PackView &v, cudaStream_t st, StepSrc step, bool ene
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
       }
       if (energy_only)
-        PDGPU_LAUNCH(k_lcpo_cand_tiles<true>, 8 * sms, 128, 0, st, v, step);
+        PDGPU_LAUNCH_DEP(k_lcpo_cand_tiles<true>, 8 * sms, 128, 0, st, v, step);
       else
-        PDGPU_LAUNCH(k_lcpo_cand_tiles<false>, 8 * sms, 128, 0, st, v, step);
+        PDGPU_LAUNCH_DEP(k_lcpo_cand_tiles<false>, 8 * sms, 128, 0, st, v, step);
     }
     if (energy_only) {
       if (from_tiles)
-        PDGPU_LAUNCH((k_lcpo_list<true, true>), blocks, tpb, 0, st, v, step);
+        PDGPU_LAUNCH_DEP((k_lcpo_list<true, true>), blocks, tpb, 0, st, v, step);
       else
-        PDGPU_LAUNCH((k_lcpo_list<true, false>), blocks, tpb, 0, st, v, step);
+        PDGPU_LAUNCH_DEP((k_lcpo_list<true, false>), blocks, tpb, 0, st, v, step);
     } else {
       if (from_tiles)
-        PDGPU_LAUNCH((k_lcpo_list<false, true>), blocks, tpb, 0, st, v, step);
+        PDGPU_LAUNCH_DEP((k_lcpo_list<false, true>), blocks, tpb, 0, st, v, step);
       else
-        PDGPU_LAUNCH((k_lcpo_list<false, false>), blocks, tpb, 0, st, v, step);
+        PDGPU_LAUNCH_DEP((k_lcpo_list<false, false>), blocks, tpb, 0, st, v, step);
     }
   } else {
     if (energy_only)
-      PDGPU_LAUNCH(k_lcpo_eval<true>, blocks, tpb, 0, st, v, step);
+      PDGPU_LAUNCH_DEP(k_lcpo_eval<true>, blocks, tpb, 0, st, v, step);
     else
-      PDGPU_LAUNCH(k_lcpo_eval<false>, blocks, tpb, 0, st, v, step);
+      PDGPU_LAUNCH_DEP(k_lcpo_eval<false>, blocks, tpb, 0, st, v, step);
   }
 }
 void launch_lcpo(const PackView &v, cudaStream_t st, StepSrc step, bool energy_only, bool from_tiles) {
