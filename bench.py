@@ -76,10 +76,10 @@ METRIC = "GB MD ns/day"
 # of the 20,566-atom MD workload (dram__bytes_read.sum + dram__bytes_write.sum,
 # cold caches: 1,924,864 + 3,327,488 + 3,181,312 bytes read, nothing written);
 # ncu cannot run inside the timed bench, so the figure is carried here
-NCU_TRAFFIC_EVAL = 8433664
+NCU_TRAFFIC_EVAL = 8333888
 # warp instructions the same three launches executed (smsp__inst_executed.sum
 # of that capture: phases A, B, C), for the issue roof beside the FP32/SFU one
-NCU_INST_EVAL = (5630203, 14581779, 6049203)
+NCU_INST_EVAL = (5550526, 13871051, 5805610)
 
 
 def rank_info():
