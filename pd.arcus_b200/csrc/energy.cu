@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energy(PackView v, int mode,
       if (done == v.n_sys - 1) {
         step_dev[2] = 0;
         if ((mode & EM_GATE) && (__ldcg(&v.flags[F_NAN]) || __ldcg(&v.flags[F_LCPO_CAND])))
-          atomicExch(&v.flags[F_NL_OVERFLOW], 2);
+          atomicExch(&v.flags[F_NL_OVERFLOW], kGateShut);
         __threadfence();
         atomicAdd(&step_dev[0], 1);
       }

@@ -90,7 +90,7 @@ enum EnergyMode {
   EM_BONDED = 8,       // bond, angle, torsion, bond virial
   EM_KINETIC = 16,     // ekin, etot
   EM_RECORD = 32,      // history row + step counter advance (step loops)
-  EM_GATE = 512,       // with EM_RECORD: F_NL_OVERFLOW = 2 after a NaN or F_LCPO_CAND (the next block skips)
+  EM_GATE = 512,       // with EM_RECORD: F_NL_OVERFLOW = kGateShut after a NaN or F_LCPO_CAND (the next block skips)
   EM_ASSIGN = 64,      // form the record from zero (its slots were not zeroed before the step)
   EM_SURF = 128,       // LCPO surface term: epot_surf
   EM_PAIR_GB_SLOW = 256  // GB with FastMode off (calcBornForces): pol + self added to epot alone;
@@ -251,6 +251,13 @@ struct PackView {
 // F_LCPO_CAND: an atom had more LCPO overlap candidates than a warp sorts
 // F_BARRIER: a grid barrier of the evaluation kernel ran out of time
 enum Flag { F_NL_OVERFLOW = 0, F_NAN = 1, F_CELL_CLAMP = 2, F_LCPO_CAND = 3, F_BARRIER = 4, F_COUNT = 8 };
+// F_NL_OVERFLOW: 1, the last rebuild did not fit its buffers (the steps after
+// it do nothing until the host has grown them); kGateShut, the MD period
+// before this one ended in an error (EM_GATE): this one's steps do nothing
+// either, and its rebuild leaves the pair structure of the failed period as
+// it is (the list rows, the tiles and xs; the cell grid and the sort are a
+// rebuild's own scratch), so that what the caller evaluates next finds it.
+constexpr int kGateShut = 2;
 constexpr const char *kLcpoCandMsg =
     "an atom has more than 256 LCPO overlap candidates (atoms closer than their radii + 2.8 A)";
 // per system: a tile pass met a non-finite pair term (its fixed-point sums
@@ -418,7 +425,7 @@ void launch_gb_chain(const PackView &v, cudaStream_t st);
 // launchers above pick them when v.tile_mode is set.  tile_launch_shapes
 // sets v.tile_blocks (host only: an occupancy query per pass kernel).
 void tile_launch_shapes(PackView &v);
-void launch_tiles_build(const PackView &v, cudaStream_t st);
+void launch_tiles_build(const PackView &v, cudaStream_t st, bool filled = false);
 // the tiles straight from the positions (no list); every system of the pack
 // at most kTileSearchMaxAtoms atoms (the search tests every j-cluster box of
 // a system against each of its i-clusters)

@@ -310,6 +310,9 @@ constexpr int kScanWarps = 8;
 template <bool FILL, bool FUSED>
 __global__ void __launch_bounds__(32 * kScanWarps) k_nlist_scan(PackView v) {
   PDGPU_DEP_ENTRY();
+  if (v.flags[F_NL_OVERFLOW] == kGateShut) return;
+  // the tiles are made again from the rows (launch_tiles_build)
+  if (FILL && v.tile_mode && blockIdx.x == 0 && threadIdx.x < 2) v.tile_count[threadIdx.x] = 0;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   long long out = 0;
@@ -527,8 +530,9 @@ __global__ void __launch_bounds__(kSmallThreads) k_cells_small(PackView v) {
 
 // --------------------------------------------------------------- scans
 // exclusive scan of row_cnt (int) into row_start (int64), total at [n]
-__global__ void k_scan_blocks(const int *cnt, int n, long long *out, long long *bsum) {
+__global__ void k_scan_blocks(const int *flags, const int *cnt, int n, long long *out, long long *bsum) {
   PDGPU_DEP_ENTRY();
+  if (flags[F_NL_OVERFLOW] == kGateShut) return;
   __shared__ long long sh[1024];
   int t = threadIdx.x;
   int idx = blockIdx.x * 1024 + t;
@@ -545,8 +549,9 @@ __global__ void k_scan_blocks(const int *cnt, int n, long long *out, long long *
   if (t == 1023) bsum[blockIdx.x] = sh[t];
 }
 
-__global__ void k_scan_bsum(long long *bsum, int nb, long long *total_out) {
+__global__ void k_scan_bsum(const int *flags, long long *bsum, int nb, long long *total_out) {
   PDGPU_DEP_ENTRY();
+  if (flags[F_NL_OVERFLOW] == kGateShut) return;
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     long long run = 0;
     for (int k = 0; k < nb; k++) {
@@ -558,14 +563,16 @@ __global__ void k_scan_bsum(long long *bsum, int nb, long long *total_out) {
   }
 }
 
-__global__ void k_scan_add(long long *out, int n, const long long *bsum) {
+__global__ void k_scan_add(const int *flags, long long *out, int n, const long long *bsum) {
   PDGPU_DEP_ENTRY();
+  if (flags[F_NL_OVERFLOW] == kGateShut) return;
   int idx = blockIdx.x * 1024 + threadIdx.x;
   if (idx < n) out[idx] += bsum[blockIdx.x];
 }
 
 __global__ void k_set_overflow(PackView v) {
   PDGPU_DEP_ENTRY();
+  if (v.flags[F_NL_OVERFLOW] == kGateShut) return;
   if (v.row_start[v.n_atoms] > v.nl_cap) atomicExch(&v.flags[F_NL_OVERFLOW], 1);
 }
 
@@ -602,9 +609,9 @@ void launch_nlist_count(Pack &p, cudaStream_t st) {
   PDGPU_LAUNCH_DEP(k_cell_ranges, (N + 255) / 256, 256, 0, st, v.cell_key, N, v.cell_start, v.cell_end);
   PDGPU_LAUNCH_DEP((k_nlist_scan<false, false>), (N + kScanWarps - 1) / kScanWarps, 32 * kScanWarps, 0, st, v);
   int nb = (N + 1023) / 1024;
-  PDGPU_LAUNCH_DEP(k_scan_blocks, nb, 1024, 0, st, v.row_cnt, N, v.row_start, p.scan_tmp);
-  PDGPU_LAUNCH_DEP(k_scan_bsum, 1, 32, 0, st, p.scan_tmp, nb, v.row_start + N);
-  PDGPU_LAUNCH_DEP(k_scan_add, nb, 1024, 0, st, v.row_start, N, p.scan_tmp);
+  PDGPU_LAUNCH_DEP(k_scan_blocks, nb, 1024, 0, st, v.flags, v.row_cnt, N, v.row_start, p.scan_tmp);
+  PDGPU_LAUNCH_DEP(k_scan_bsum, 1, 32, 0, st, v.flags, p.scan_tmp, nb, v.row_start + N);
+  PDGPU_LAUNCH_DEP(k_scan_add, nb, 1024, 0, st, v.flags, v.row_start, N, p.scan_tmp);
   PDGPU_LAUNCH_DEP(k_set_overflow, 1, 1, 0, st, v);
 }
 
@@ -614,7 +621,7 @@ void launch_nlist_fill(Pack &p, cudaStream_t st) {
   if (N == 0) return;
   PDGPU_LAUNCH_DEP((k_nlist_scan<true, false>), (N + kScanWarps - 1) / kScanWarps, 32 * kScanWarps, 0, st, v);
   // the same pair set re-cut into cluster-pair tiles for the tile passes
-  if (v.tile_mode) launch_tiles_build(v, st);
+  if (v.tile_mode) launch_tiles_build(v, st, true);
 }
 
 void launch_nlist_rebuild(Pack &p, cudaStream_t st) {
@@ -637,7 +644,7 @@ void launch_nlist_rebuild(Pack &p, cudaStream_t st) {
   PDGPU_LAUNCH_DEP(k_cells_small, 1, kSmallThreads, kSmallSmem, st, v);
   PDGPU_LAUNCH_DEP((k_nlist_scan<false, false>), blocks, 32 * kScanWarps, 0, st, v);
   PDGPU_LAUNCH_DEP((k_nlist_scan<true, true>), blocks, 32 * kScanWarps, 0, st, v);
-  if (v.tile_mode) launch_tiles_build(v, st);
+  if (v.tile_mode) launch_tiles_build(v, st, true);
 }
 
 }  // namespace pdgpu

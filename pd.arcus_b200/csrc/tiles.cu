@@ -207,6 +207,7 @@ __global__ void __launch_bounds__(128) k_tile_build(PackView v) {
 // 64 OPLS peptides 150 -> 33 us, 512 peptides 671 -> 150 us.
 __global__ void __launch_bounds__(128) k_cluster_boxes(PackView v) {
   PDGPU_DEP_ENTRY();
+  if (v.flags[F_NL_OVERFLOW] == kGateShut) return;  // (k_tile_search returns on the flag too)
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < 2) v.tile_count[t] = 0;
   const int jc = t >> 3, k = t & 7;
@@ -897,9 +898,9 @@ void tile_launch_shapes(PackView &v) {
     v.tile_blocks[p] = (int)std::max(1LL, std::min((long long)std::max(occ[p], 1) * sms, need));
   v.ev_blocks = eval_tiles_grid(v.tile_cap);
 }
-void launch_tiles_build(const PackView &v, cudaStream_t st) {
+void launch_tiles_build(const PackView &v, cudaStream_t st, bool filled) {
   if (!v.n_sc) return;
-  cudaMemsetAsync(v.tile_count, 0, 2 * sizeof(int), st);
+  if (!filled) cudaMemsetAsync(v.tile_count, 0, 2 * sizeof(int), st);
   size_t smem = tile_build_smem(v.max_sys_atoms);
   static size_t opted = 0;  // dynamic shared memory above 48 KB needs an opt-in
   if (smem > 48 * 1024 && smem > opted) {
