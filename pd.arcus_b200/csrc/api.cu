@@ -1450,7 +1450,7 @@ void pdgpu::calc_forces_enqueue(cudaStream_t st, SysEntry *e, bool reduce, StepS
   if (first) {
     cudaEventRecord(P.fork, st);
     cudaStreamWaitEvent(P.side, P.fork, 0);
-    cudaMemsetAsync(P.v.fx, 0, sizeof(long long) * 3 * (size_t)P.v.n_atoms, P.side);  // fx, fy, fz: one block
+    launch_zero_bonded(P.v, P.side);
     if (surf) {
       if (bonded) cudaEventRecord(P.fork2, P.side);
       launch_lcpo(P.v, P.side, step, false, P.csr_stale);

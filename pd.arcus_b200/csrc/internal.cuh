@@ -399,6 +399,7 @@ void launch_soa_to_aos(double *aos, const double *X, const double *Y, const doub
 // forces in N, interleaved [n][3], for the caller (scale: kcal/mol/A -> N)
 void launch_forces_out(const PackView &v, double scale, double *out, cudaStream_t st);
 void launch_zero(const PackView &v, cudaStream_t st);
+void launch_zero_bonded(const PackView &v, cudaStream_t st);
 // neighbour list: build phases.  count -> (host may read total) -> fill
 void launch_nlist_count(Pack &p, cudaStream_t st);
 void launch_nlist_fill(Pack &p, cudaStream_t st);

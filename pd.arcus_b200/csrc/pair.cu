@@ -149,6 +149,20 @@ void launch_soa_to_aos(double *aos, const double *X, const double *Y, const doub
   if (n > 0) PDGPU_LAUNCH(k_soa_to_aos, (3 * n + 255) / 256, 256, 0, st, aos, X, Y, Z, n);
 }
 
+// The bonded-force accumulators, for an evaluation whose bonded or surface
+// terms start at once (fx, fy, fz are one block).  A memset would also clear
+// the forces of a step that does nothing (the flag): they are what the caller
+// of a failed run reads.
+__global__ void k_zero_bonded(PackView v) {
+  PDGPU_DEP_ENTRY();
+  if (v.flags[F_NL_OVERFLOW]) return;
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 3 * (size_t)v.n_atoms) v.fx[i] = 0;
+}
+void launch_zero_bonded(const PackView &v, cudaStream_t st) {
+  if (v.n_atoms) PDGPU_LAUNCH_DEP(k_zero_bonded, (3 * (size_t)v.n_atoms + 255) / 256, 256, 0, st, v);
+}
+
 __global__ void k_zero(PackView v) {
   if (v.flags[F_NL_OVERFLOW]) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -510,7 +510,7 @@ Pack *pack_create(int device, cudaStream_t st, const std::vector<const SystemHos
   PALLOC(v.gx, N);
   PALLOC(v.gy, N);
   PALLOC(v.gz, N);
-  PALLOC(v.fx, 3 * (size_t)N);  // one block: zeroed by one memset
+  PALLOC(v.fx, 3 * (size_t)N);  // one block: zeroed in one go (k_zero_bonded)
   v.fy = v.fx + N;
   v.fz = v.fx + 2 * (size_t)N;
   PALLOC(v.fox, N);

@@ -129,3 +129,13 @@ def test_pairs_after_a_failed_run(kind, path, graph, gpu_ctx):
     for a, b in zip(single[3] + single[5] + (single[4],), whole[3] + whole[5] + (whole[4],)):
         np.testing.assert_array_equal(a, b)
     assert single[4][4] > 0 if path else single[5][0][-1] > 0
+
+
+# (past its ranks' limit the surface term keeps whichever candidates came first)
+@pytest.mark.parametrize("kind,path,graph", [c for c in CASES if c[:2] != ("surface", 1)])
+def test_forces_after_a_failed_run(kind, path, graph, gpu_ctx):
+    single = _failed_run(gpu_ctx, kind, path, graph, EVERY)
+    whole = _failed_run(gpu_ctx, kind, path, graph, None)
+    assert np.abs(np.nan_to_num(single[2][0])).max() > 0
+    for a, b in zip(single[2][:2], whole[2][:2]):
+        np.testing.assert_array_equal(a, b)
