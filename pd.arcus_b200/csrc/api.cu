@@ -1825,9 +1825,11 @@ static int md_run_impl(pdgpu_ctx *c, SysEntry *e, const pdgpu_md_params *p, int3
   steps0[2] = 0;
   PDGPU_CUDA(cudaMemcpyAsync(e->step_dev, steps0, sizeof(int) * 3, cudaMemcpyHostToDevice, c->st));
   cudaEventRecord(P.ev0, c->st);
-  // One block of the run's steps from s, enqueued with its flag copy.
+  // One block of the run's steps from s, enqueued with its flag copy, and the
+  // host's notes on what it leaves on the device.
   struct Block {
-    int s, n, slot;
+    int s, n, slot, last_ebuf;
+    bool csr_stale;
   };
   auto enqueue_block = [&](int s, int counter, Block *out) -> int {
     // Blocks follow the list periods (protocolbase.cpp:113-122: a rebuild
@@ -1912,6 +1914,8 @@ static int md_run_impl(pdgpu_ctx *c, SysEntry *e, const pdgpu_md_params *p, int3
     PDGPU_CUDA(cudaEventRecord(e->block_ev[out->slot], c->st));
     out->s = s;
     out->n = block;
+    out->last_ebuf = P.last_ebuf;
+    out->csr_stale = P.csr_stale;
     return PDGPU_OK;
   };
   const int counter0 = P.nlist_counter;
@@ -1941,8 +1945,10 @@ static int md_run_impl(pdgpu_ctx *c, SysEntry *e, const pdgpu_md_params *p, int3
     if ((r = barrier_check(c, P, flags))) return r;
     const bool cand = flags[F_LCPO_CAND], nan = flags[F_NAN], overflow = flags[F_NL_OVERFLOW] == 1;
     if (cand || nan || overflow) {
-      // the block behind it has done nothing
+      // the block behind it has done nothing, so this block's notes hold
       if ((r = sync_check(c, "md block"))) return r;
+      P.last_ebuf = cur.last_ebuf;
+      P.csr_stale = cur.csr_stale;
       if (cand || (nan && !overflow))  // the gate opens again
         PDGPU_CUDA(cudaMemsetAsync(v.flags + F_NL_OVERFLOW, 0, sizeof(int), c->st));
     }

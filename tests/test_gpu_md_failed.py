@@ -29,7 +29,7 @@ def _lattice(side, spacing):
 def _handle(gpu_ctx, kind):
     """(handle, closers, good positions, the run's positions, velocities, steps)"""
     import pdgpu
-    steps, vel = 35, None
+    steps, vel = 15, None  # the period behind the first is a shorter one
     if kind == "surface":
         # closing in from 4.0 A: past 2.9 A an atom has more overlap partners than the term ranks
         pos = _lattice(9, 4.0)
@@ -138,4 +138,52 @@ def test_forces_after_a_failed_run(kind, path, graph, gpu_ctx):
     whole = _failed_run(gpu_ctx, kind, path, graph, None)
     assert np.abs(np.nan_to_num(single[2][0])).max() > 0
     for a, b in zip(single[2][:2], whole[2][:2]):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("kind,path,graph", [c for c in CASES if c[0] != "surface"])
+def test_atom_energies_after_a_failed_run(kind, path, graph, gpu_ctx):
+    """Odd and even steps keep them in two buffers: the failed period's last
+    step decides, not that of the period behind."""
+    single = _failed_run(gpu_ctx, kind, path, graph, EVERY)
+    whole = _failed_run(gpu_ctx, kind, path, graph, None)
+    assert np.abs(np.nan_to_num(single[2][2])).max() > 0
+    np.testing.assert_array_equal(single[2][2], whole[2][2])
+
+
+def _peptide(gpu_ctx, path):
+    arrays, meta = load_library("lib16_opls_s4")[7]
+    ws, ff = build_workspace(arrays, meta, gpu_ctx)
+    assert ws.setPairPath(path) == path
+    return ws, ff, np.ascontiguousarray(arrays["pos"])
+
+
+def _md(gpu_ctx, ws, first, steps, graph=1):
+    from pdgpu import _abi as A
+    p = A.md_params_default()
+    p.Integrator, p.UpdateNList, p.UseGraph = A.INTEGRATOR_VELOCITY_VERLET, EVERY, graph
+    p.Timestep, p.Seed = 1e-15, 3
+    return A.lib().pdgpu_md_run(gpu_ctx.ptr, ws._sys, ctypes.byref(p), first, steps, 100, None)
+
+
+@pytest.mark.parametrize("path", [0, 1])
+def test_list_of_a_run_that_failed_inside_a_period(path, gpu_ctx):
+    """The run starts inside a period on a list made for it (no tile search at
+    these positions) and fails there; the period behind would have searched."""
+    from pdgpu import _abi as A
+    lists = []
+    for steps in (5, 25):
+        ws, ff, pos = _peptide(gpu_ctx, path)
+        ws.nlist().calcNewList()
+        assert _md(gpu_ctx, ws, 0, 5) == 0
+        moved = 1.05 * pos
+        bad = moved.copy()
+        bad[10] = np.nan
+        A.check(A.lib().pdgpu_set_positions(gpu_ctx.ptr, ws._sys, A.dptr(bad)))
+        A.check(A.lib().pdgpu_system_set_params(gpu_ctx.ptr, ws._sys, ctypes.byref(ff._nb()._params())))
+        assert _md(gpu_ctx, ws, 5, steps) != 0
+        A.check(A.lib().pdgpu_set_positions(gpu_ctx.ptr, ws._sys, A.dptr(moved)))
+        lists.append(ws.nlist().getData(shadow=True))
+        ws.close()
+    for a, b in zip(*lists):
         np.testing.assert_array_equal(a, b)
