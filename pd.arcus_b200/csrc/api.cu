@@ -1620,11 +1620,13 @@ int pdgpu_md_init_velocities(pdgpu_ctx *c, int32_t sys, double temperature, uint
 // one MD step enqueue: forces, integrate, one energy reduction that also
 // records the step and advances the device step counter (7 launches)
 }  // extern "C"
+// The energy buffer of step q of a block.
+static int step_ebuf(const Pack &P, int q) { return (P.v.tile_mode && !P.slow()) ? (q & 1) : 0; }
 void pdgpu::md_step_enqueue(cudaStream_t st, SysEntry *e, const MDCoef &k, int q, bool gate) {
   Pack &P = *e->pack;
   StepSrc step;
   step.p = e->step_dev;  // MolecularDynamics::run_core sets WorkSpace::Step = Step (md.cpp:214)
-  const int b = (P.v.tile_mode && !P.slow()) ? (q & 1) : 0;  // this step's energy buffer
+  const int b = step_ebuf(P, q);
   EvalOpts o;
   o.ebuf = b;
   o.coop = P.coop_md ? 1 : 0;
@@ -1906,7 +1908,9 @@ static int md_run_impl(pdgpu_ctx *c, SysEntry *e, const pdgpu_md_params *p, int3
       PDGPU_CUDA(cudaGraphLaunch(g->exec, c->st));
       launch_counter() += g->nodes;
       e->graph_replays++;
-      if (rebuild) P.csr_stale = tile_search_ok(P);  // what the graph's rebuild made
+      // what a replay's rebuild made and which buffer its last step used
+      if (rebuild) P.csr_stale = tile_search_ok(P);
+      P.last_ebuf = step_ebuf(P, block - 1);
     }
     if (s + block >= steps) cudaEventRecord(P.ev1, c->st);
     PDGPU_CUDA(cudaMemcpyAsync(e->pin_flags + out->slot * F_COUNT, v.flags, sizeof(int) * F_COUNT,

@@ -187,3 +187,25 @@ def test_list_of_a_run_that_failed_inside_a_period(path, gpu_ctx):
         ws.close()
     for a, b in zip(*lists):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("steps", [10, 5])
+def test_atom_energies_after_a_replayed_period(steps, gpu_ctx):
+    """A period replayed from its graph, with a single evaluation before it."""
+    from pdgpu import _abi as A
+    out = []
+    for graph in (1, 0):
+        ws, ff, pos = _peptide(gpu_ctx, 1)
+        ws.nlist().calcNewList()
+        for k in range(2):
+            assert _md(gpu_ctx, ws, 10 * k, steps, graph) == 0
+            if steps < EVERY:  # the rest of the period, so the next call begins one
+                assert _md(gpu_ctx, ws, 10 * k + steps, EVERY - steps - 1, graph) == 0
+                assert _md(gpu_ctx, ws, 10 * k + EVERY - 1, 1, graph) == 0
+            if k == 0:
+                A.check(A.lib().pdgpu_calc_forces(gpu_ctx.ptr, ws._sys))
+        if steps < EVERY:
+            assert _md(gpu_ctx, ws, 20, steps, graph) == 0
+        out.append(_state(A.lib(), gpu_ctx.ptr, ws._sys, len(pos))[2])
+        ws.close()
+    np.testing.assert_array_equal(*out)
