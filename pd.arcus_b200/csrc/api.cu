@@ -1859,12 +1859,15 @@ static int md_run_impl(pdgpu_ctx *c, SysEntry *e, const pdgpu_md_params *p, int3
         break;
       }
       // graphs are cached per system; the key holds every value baked in
+      // (without a rebuild of its own, where the surface term's candidates
+      // come from: the tiles, or the list rows where these are as new)
+      const int surf_rows = !rebuild && P.v.lc.update > 0 && !P.csr_stale;
       char key[288];
-      snprintf(key, sizeof key, "%d|%d|%p|%lld|%p|%d|%d|%.17g|%.17g|%.17g|%d|%d|%d|%d%d%d|%d%d%d|%p|%d|%d", block,
+      snprintf(key, sizeof key, "%d|%d|%p|%lld|%p|%d|%d|%.17g|%.17g|%.17g|%d|%d|%d|%d%d%d|%d%d%d|%p|%d|%d|%d", block,
                (int)rebuild, (void *)v.nl, v.nl_cap, (void *)e->hist, k.integrator, k.steps, k.dt, k.gamma,
                k.temp, k.stochastic_h, P.radix_passes, (int)e->host->params.FastMode, v.lpa[0], v.lpa[1],
                v.lpa[2], v.tile_mode, (int)tile_search_ok(P), (int)P.coop_md, (void *)e->traj_dev, e->traj_every,
-               e->traj_dev_cap);
+               e->traj_dev_cap, surf_rows);
       SysEntry::GraphSlot *g = nullptr;
       for (auto &q : e->gslots)
         if (q.key == key) g = &q;

@@ -273,3 +273,44 @@ def test_lcpo_large_system(gpu_ctx):
     assert np.array_equal(area, o_area)
     assert np.array_equal(deriv, o_deriv)
     ws.close()
+
+
+def test_lcpo_in_a_replayed_period(gpu_ctx):
+    """A stretch without a rebuild, captured when an export had just made the
+    list rows and replayed when the tiles are newer: the overlap candidates
+    come from the tiles then.  Against the same calls without graphs."""
+    from conftest import build_workspace
+    from test_gpu_edge import _system
+    import pdgpu
+    from pdgpu import _abi as A
+    g = np.arange(7)
+    pos = 4.5 * np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3).astype(np.float64)
+    rng = np.random.default_rng(11)
+    pos += rng.normal(0.0, 0.1, pos.shape)
+    moved = np.ascontiguousarray(pos[rng.permutation(len(pos))])
+    arrays, meta = _system(pos, np.arange(len(pos)) % 300)
+    arrays.update(lcpo_radius=np.full(len(pos), 3.2), lcpo_use=np.ones(len(pos), np.uint8),
+                  lcpo_p=np.tile([0.5, -0.3, -0.001, 0.0005], (len(pos), 1)))
+    out = []
+    for graph in (1, 0):
+        ws, ff = build_workspace(arrays, meta, gpu_ctx)
+        sasa = pdgpu.FF_SASA_LCPO(ws)
+        sasa.GlobalASP, sasa.UpdateSasa = 0.005, 1
+        ff.add(sasa)
+        ff.ensuresetup()
+        ws.setPairPath(1)
+        ws.nlist().calcNewList()
+        p = A.md_params_default()
+        p.Integrator, p.UpdateNList, p.UseGraph = A.INTEGRATOR_VELOCITY_VERLET, 10, graph
+        p.Timestep, p.Seed = 1e-15, 3
+        for k in range(4):
+            if k == 1:
+                ws.nlist().getData(shadow=True)
+            if k == 2:
+                A.check(A.lib().pdgpu_set_positions(gpu_ctx.ptr, ws._sys, A.dptr(moved)))
+            A.check(A.lib().pdgpu_md_run(gpu_ctx.ptr, ws._sys, ctypes.byref(p), 5 * k, 5, 20, None))
+        out.append(sasa.sasa() + (ws._pull_forces().copy(),))
+        ws.close()
+    assert np.abs(out[1][1]).max() > 0
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
