@@ -1928,18 +1928,27 @@ static int md_run_impl(pdgpu_ctx *c, SysEntry *e, const pdgpu_md_params *p, int3
   const int counter0 = P.nlist_counter;
   int done = 0, enqueued = 0, nrun = 0, attempt = 0, slot = 0;  // steps done and enqueued, blocks in flight
   Block run[2];                                                 // oldest first
+  // Leaves with an error of the call itself, blocks in flight or not: one of
+  // them may have set the flag that makes every later evaluation do nothing
+  // (and, when it overflowed, the list rows do not fit their buffer).
+  auto leave = [&](int error) {
+    int f = 0;
+    cudaStreamSynchronize(c->st);
+    if (cudaMemcpy(&f, v.flags + F_NL_OVERFLOW, sizeof f, cudaMemcpyDeviceToHost) == cudaSuccess && f) {
+      if (f != kGateShut) P.have_list = false;
+      cudaMemset(v.flags + F_NL_OVERFLOW, 0, sizeof f);
+    }
+    return error;
+  };
   while (done < steps) {
     while (nrun < (e->traj_every <= 0 && !P.coop_md ? 2 : 1) && enqueued < steps) {
       run[nrun].slot = slot ^= 1;
-      if ((r = enqueue_block(enqueued, counter0 + enqueued, &run[nrun]))) {
-        cudaStreamSynchronize(c->st);
-        return r;
-      }
+      if ((r = enqueue_block(enqueued, counter0 + enqueued, &run[nrun]))) return leave(r);
       enqueued += run[nrun++].n;
     }
     const Block cur = run[0];
     const bool last = cur.s + cur.n >= steps;
-    if (last && tail && (r = tail())) return r;
+    if (last && tail && (r = tail())) return leave(r);
     if (last) {
       r = sync_check(c, "md block");
     } else {
@@ -1949,7 +1958,7 @@ static int md_run_impl(pdgpu_ctx *c, SysEntry *e, const pdgpu_md_params *p, int3
     }
     if (r) return r;
     const int *flags = e->pin_flags + cur.slot * F_COUNT;
-    if ((r = barrier_check(c, P, flags))) return r;
+    if ((r = barrier_check(c, P, flags))) return leave(r);
     const bool cand = flags[F_LCPO_CAND], nan = flags[F_NAN], overflow = flags[F_NL_OVERFLOW] == 1;
     if (cand || nan || overflow) {
       // the block behind it has done nothing, so this block's notes hold
