@@ -1238,30 +1238,26 @@ int pdgpu_gb_energies(pdgpu_ctx *c, int32_t sys) {
   int r = need_csr(c, e);
   if (r) return r;
   // calcEnergies: radii, FF_NonBonded::calcEnergies at Dielectric =
-  // DielectricSolute (gbff.cpp:44), then calcBornEnergy.  The settings move
-  // to the device and back only where that dielectric is not the system's own
-  // already (the components' setup makes it so).
+  // DielectricSolute (gbff.cpp:44), then calcBornEnergy.  These settings move
+  // to the device and the pack's own back only where they differ (the
+  // components' setup makes that dielectric the system's own already).
   const int S = e->nsys();
-  bool own = true;
-  for (int s = 0; s < S; s++) own = own && e->members[s]->params.Dielectric == e->members[s]->params.DielectricSolute;
-  std::vector<SysParams> saved;
-  if (!own) {
-    saved = P.sp;
-    for (int s = 0; s < S; s++) {
-      pdgpu_ff_params q = e->members[s]->params;
-      q.Dielectric = q.DielectricSolute;
-      pack_set_params(&P, s, q);
-    }
-    PDGPU_CUDA(cudaMemcpyAsync((void *)P.v.sp, P.sp.data(), sizeof(SysParams) * S, cudaMemcpyHostToDevice, c->st));
+  std::vector<SysParams> at(S);
+  for (int s = 0; s < S; s++) {
+    pdgpu_ff_params q = e->members[s]->params;
+    q.Dielectric = q.DielectricSolute;
+    at[s] = make_sys_params(q);
   }
+  const size_t bytes = sizeof(SysParams) * S;
+  const bool own = memcmp(at.data(), P.sp.data(), bytes) == 0;
+  if (!own) PDGPU_CUDA(cudaMemcpyAsync((void *)P.v.sp, at.data(), bytes, cudaMemcpyHostToDevice, c->st));
   launch_born_radii(P.v, c->st);
-  launch_nonbonded(P.v, c->st, P.sp[0].elec_mode);
+  launch_nonbonded(P.v, c->st, at[0].elec_mode);
   launch_born_energy(P.v, c->st);
   launch_energy(P.v, c->st, EM_PAIR_NB | EM_BORN_ENERGY);
   r = sync_check(c, "gb_energies");
   if (own) return r;
-  P.sp = saved;
-  PDGPU_CUDA(cudaMemcpyAsync((void *)P.v.sp, P.sp.data(), sizeof(SysParams) * S, cudaMemcpyHostToDevice, c->st));
+  PDGPU_CUDA(cudaMemcpyAsync((void *)P.v.sp, P.sp.data(), bytes, cudaMemcpyHostToDevice, c->st));
   int r2 = sync_check(c, "gb_energies");
   return r ? r : r2;
 }

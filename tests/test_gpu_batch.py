@@ -202,3 +202,29 @@ def test_batch_minimise_matches_alone(gpu_ctx):
         assert taken[s] == alone_taken[s] == 30
         assert np.array_equal(b.split(pos)[s], alone_pos[s])
     b.close()
+
+
+def test_batch_energies_after_a_members_settings_change(gpu_ctx):
+    """The energies-only call works at the solute's dielectric; here the batch
+    was made with another and the member's settings then get the solute's (the
+    batch keeps its own): the energies are those of a batch made with it."""
+    import pdgpu
+    from pdgpu import _abi as A
+    L = A.lib()
+    got = []
+    for made_with in (10.0, 1.0):
+        (ws, ff, a, m), = _library(gpu_ctx, "lib16_amber_s3", 1)
+        p = ff._nb()._params()
+        assert p.DielectricSolute == 1.0
+        p.Dielectric = made_with
+        A.check(L.pdgpu_system_set_params(gpu_ctx.ptr, ws._sys, ctypes.byref(p)))
+        b = pdgpu.Batch([ws])
+        p.Dielectric = p.DielectricSolute
+        A.check(L.pdgpu_system_set_params(gpu_ctx.ptr, ws._sys, ctypes.byref(p)))
+        b.calcNewList()
+        A.check(L.pdgpu_gb_energies(gpu_ctx.ptr, b._id))
+        got.append(b.energies().copy())
+        b.close()
+        ws.close()
+    assert np.abs(got[1]).max() > 0
+    np.testing.assert_array_equal(*got)
