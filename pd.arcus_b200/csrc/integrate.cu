@@ -125,18 +125,25 @@ __global__ void k_vel_scale(PackView v, double kB, double temp, double kcal2J_pe
 }
 
 // --------------------------------------------------------------- minimiser
-// CG dot products: per (chunk, system) partials of fmagold = sum of.of and
-// fmagnew = sum (of-f).f into e_part slots 0 and 1; the last block of each
-// system adds them in a fixed order into its state, before the energy record
-// whose last block takes the step's decision (min_control).
-__global__ void k_min_dots(PackView v, MinState *ms, double N_per_unit, int C) {
-  PDGPU_DEP_ENTRY();
-  if (v.flags[F_NL_OVERFLOW]) return;
+// CG dot products: per (256-atom chunk, system) partials of fmagold = sum of
+// of.of and fmagnew = sum of (of-f).f; the last block of each system to finish
+// adds them in a fixed order into its state, before the energy record whose
+// last block takes the step's decision (min_control).  An atom per thread: a
+// step waits for this launch and its blocks for twelve loads an atom, which
+// the record's 4,096-item chunks made sixteen times in a row.  A step's share
+// (CG step minus SD step), 4,096 items -> 256: 506 atoms 7.2 -> 4.0 us, 2,972
+// 14.2 -> 3.6, 20,566 17.2 -> 5.5.  A system of one chunk needs no second stage.
+constexpr int kDotChunk = 256;
+static_assert(2 * (kReduceChunk / kDotChunk) <= kPartSlots, "two partials a chunk fit the reduction buffer");
+__global__ void __launch_bounds__(kDotChunk) k_min_dots(PackView v, MinState *ms, double N_per_unit, int C) {
   const int c = blockIdx.x, s = blockIdx.y;
-  int a0 = v.atom_off[s] + c * kReduceChunk, a1 = min(a0 + kReduceChunk, v.atom_off[s + 1]);
-  __shared__ double sa[256], sb[256];
+  const int i = v.atom_off[s] + c * kDotChunk + threadIdx.x, end = v.atom_off[s + 1];
+  const int mine = (end - v.atom_off[s] + kDotChunk - 1) / kDotChunk;  // this system's chunks
+  PDGPU_DEP_ENTRY();
+  if (v.flags[F_NL_OVERFLOW] || c >= mine) return;
+  __shared__ double sa[kDotChunk], sb[kDotChunk];
   double A = 0, B = 0;
-  for (int i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
+  if (i < end) {
     double f[3] = {force_N(v.fx[i], v.gx[i], v.hx[i]) * N_per_unit, force_N(v.fy[i], v.gy[i], v.hy[i]) * N_per_unit,
                    force_N(v.fz[i], v.gz[i], v.hz[i]) * N_per_unit};
     double of[3] = {v.fox[i], v.foy[i], v.foz[i]};
@@ -146,31 +153,38 @@ __global__ void k_min_dots(PackView v, MinState *ms, double N_per_unit, int C) {
   sa[threadIdx.x] = A;
   sb[threadIdx.x] = B;
   __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
+  for (int w = kDotChunk / 2; w > 0; w >>= 1) {
     if (threadIdx.x < w) {
       sa[threadIdx.x] += sa[threadIdx.x + w];
       sb[threadIdx.x] += sb[threadIdx.x + w];
     }
     __syncthreads();
   }
-  double *part = v.e_part + (size_t)s * C * 10;
+  if (mine == 1) {
+    if (threadIdx.x == 0) {
+      ms[s].fmagold = sa[0];
+      ms[s].fmagnew = sb[0];
+    }
+    return;
+  }
+  double *part = v.e_part + (size_t)s * C * 2;
   if (threadIdx.x == 0) {
-    part[(size_t)c * 10] = sa[0];
-    part[(size_t)c * 10 + 1] = sb[0];
+    part[2 * (size_t)c] = sa[0];
+    part[2 * (size_t)c + 1] = sb[0];
   }
   // the last block of the system adds the chunk partials (lanes strided over
   // the chunks, then a fixed shuffle tree)
   __shared__ int last;
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&v.e_done[s], 1) == C - 1;
+  if (threadIdx.x == 0) last = atomicAdd(&v.e_done[s], 1) == mine - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp < 2) {
     double t = 0.0;
-    for (int q = lane; q < C; q += 32) t += __ldcg(part + (size_t)q * 10 + warp);
+    for (int q = lane; q < mine; q += 32) t += __ldcg(part + 2 * (size_t)q + warp);
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (lane == 0) (warp == 0 ? ms[s].fmagold : ms[s].fmagnew) = t;
   }
@@ -305,8 +319,8 @@ MinCtl min_ctl(void *ms, int algorithm, double slope_kcal, double strict_kcal, i
 }
 void launch_min_dots(const PackView &v, cudaStream_t st, const MinCtl &c) {
   if (c.algorithm != PDGPU_MIN_CONJUGATE_GRADIENTS) return;
-  const int C = v.e_chunks;
-  PDGPU_LAUNCH_DEP(k_min_dots, dim3(C, v.n_sys), 256, 0, st, v, c.ms, consts().N_per_kcalmolA, C);
+  const int C = (v.max_sys_atoms + kDotChunk - 1) / kDotChunk;
+  if (C) PDGPU_LAUNCH_DEP(k_min_dots, dim3(C, v.n_sys), kDotChunk, 0, st, v, c.ms, consts().N_per_kcalmolA, C);
 }
 void launch_min_update(const PackView &v, cudaStream_t st, const MinCtl &c, double step_size) {
   if (v.n_atoms)

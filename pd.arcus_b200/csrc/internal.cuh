@@ -38,7 +38,7 @@ constexpr double kInvForceScale = 1.0 / 4294967296.0;
 constexpr double kJScale = 16777216.0;                // 2^24: tile pass forces and energies
 constexpr double kInvJScale = 1.0 / 16777216.0;
 constexpr int kReduceChunk = 4096;                    // items per block of the per-system reductions
-constexpr int kPartSlots = 12;                        // reduction partials per (chunk, system)
+constexpr int kPartSlots = 32;                        // reduction partials per (chunk, system), at most
 constexpr int kLcpoMax = 80;                          // overlap partners kept per atom (lcpo.h Nlistmax)
 constexpr int kLcpoCand = 256;                        // overlap candidates an atom may have (ranked, then cut to 80)
 constexpr double kBornScale = 1099511627776.0;        // 2^40
