@@ -51,40 +51,60 @@ __global__ void k_md_step(PackView v, MDDev d, const double *normals, const int 
 
 // Kinetic energies from the current velocities: every atom's (J) and each
 // system's total into its record, as an energy record with kinetic energies
-// alone would leave it.  One block per system.  The total scales the initial
-// velocities, so its order of addition is part of every trajectory: 256-atom
-// chunks (a shuffle tree per 32 atoms, the eight in order), then lane l of a
-// warp the chunks l, l + 32, ... and a shuffle tree.  Four chunks run at a
-// time; one launch takes the place of two (2.7 + 16 -> 6.4 us, 64 peptides).
-constexpr int kKinChunk = 256, kKinAtOnce = 4;
-__global__ void __launch_bounds__(kKinChunk *kKinAtOnce) k_kinetic_record(PackView v, double J2kcalmol) {
-  __shared__ double sh[kKinChunk * kKinAtOnce / 32];
-  const int s = blockIdx.x, a0 = v.atom_off[s], a1 = v.atom_off[s + 1];
+// alone would leave it.  The total scales the initial velocities, so its order
+// of addition is part of every trajectory: 256-atom chunks (a shuffle tree per
+// 32 atoms, the eight in order), then lane l of a warp the chunks l, l + 32,
+// ... and a shuffle tree.  A block takes 16 chunks, four atoms a thread at
+// once; a larger system's blocks leave their chunks' sums to its last one.
+// Bound by latency.  A call of pdgpu_md_init_velocities (four kernels and a
+// synchronisation), one block walking a system / this form: 2,972 atoms 31 / 30
+// us, 20,566 57 / 32, 97,336 183 / 33, 512,000 850 / 50; 256 peptides 36 / 35.
+constexpr int kKinChunk = 256, kKinThreads = 1024;
+constexpr int kKinChunks = kReduceChunk / kKinChunk, kKinItems = kReduceChunk / kKinThreads;
+static_assert(kKinChunks <= kPartSlots && kKinChunks <= 32, "a block's sums fit its partials and a warp");
+__global__ void __launch_bounds__(kKinThreads) k_kinetic_record(PackView v, double J2kcalmol, int C) {
+  __shared__ double sh[kReduceChunk / 32];
+  const int s = blockIdx.y, a1 = v.atom_off[s + 1], a0 = v.atom_off[s], b = a0 + blockIdx.x * kReduceChunk;
+  const int mine = (a1 - a0 + kReduceChunk - 1) / kReduceChunk;  // this system's blocks
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool skip = v.flags[F_NL_OVERFLOW];  // the record keeps its state
-  double acc = 0.0;
-  for (int b = a0, c = 0; b < a1; b += kKinChunk * kKinAtOnce, c += kKinAtOnce) {
-    const int i = b + threadIdx.x;
-    double ke = 0.0;
+  if ((int)blockIdx.x >= mine) return;
+  double ke[kKinItems];
+#pragma unroll
+  for (int r = 0; r < kKinItems; r++) {
+    const int i = b + r * kKinThreads + (int)threadIdx.x;
+    ke[r] = 0.0;
     if (i < a1) {
       const double vx = v.vx[i], vy = v.vy[i], vz = v.vz[i];
-      ke = 0.5 * v.mass_si[i] * (vx * vx + vy * vy + vz * vz);
-      v.e_atom[(size_t)AE_KIN * v.n_atoms + i] = ke;
+      ke[r] = 0.5 * v.mass_si[i] * (vx * vx + vy * vy + vz * vz);
+      v.e_atom[(size_t)AE_KIN * v.n_atoms + i] = ke[r];
     }
-    for (int o = 16; o > 0; o >>= 1) ke += __shfl_xor_sync(0xffffffffu, ke, o);
-    if (lane == 0) sh[warp] = ke;
-    __syncthreads();
-    if (warp == 0) {
-      const int q = (lane - c) & 31;  // chunk c + q goes to lane (c + q) % 32
-      if (q < kKinAtOnce) {
-        double t = 0.0;
-        for (int w = 0; w < kKinChunk / 32; w++) t += sh[q * (kKinChunk / 32) + w];
-        if (b + q * kKinChunk < a1) acc += t;
-      }
-    }
-    __syncthreads();
   }
-  if (warp != 0 || skip) return;
+#pragma unroll
+  for (int r = 0; r < kKinItems; r++) {
+    for (int o = 16; o > 0; o >>= 1) ke[r] += __shfl_xor_sync(0xffffffffu, ke[r], o);
+    if (lane == 0) sh[r * (kKinThreads / 32) + warp] = ke[r];
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  double acc = 0.0;
+  if (lane < kKinChunks)
+    for (int w = 0; w < kKinChunk / 32; w++) acc += sh[lane * (kKinChunk / 32) + w];  // (past the end: zeros)
+  if (mine > 1) {
+    double *part = v.e_part + (size_t)s * C * kKinChunks;
+    if (lane < kKinChunks) part[(size_t)blockIdx.x * kKinChunks + lane] = acc;
+    __threadfence();
+    __syncwarp();
+    int last = 0;
+    if (lane == 0) last = atomicAdd(&v.e_done[s], 1) == mine - 1;
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    __threadfence();
+    acc = 0.0;
+#pragma unroll 4
+    for (int q = lane; q < mine * kKinChunks; q += 32) acc += __ldcg(part + q);
+    if (lane == 0) v.e_done[s] = 0;
+  }
+  if (skip) return;
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if (lane) return;
   double *E = v.ene + (size_t)s * E_COUNT;
@@ -296,7 +316,8 @@ long long end_capture_count() {
 void launch_ke_from_velocities(const PackView &v, cudaStream_t st) {
   if (!v.n_atoms) return;
   const Consts &k = consts();
-  PDGPU_LAUNCH(k_kinetic_record, v.n_sys, kKinChunk * kKinAtOnce, 0, st, v, k.J2kcal * k.Na);
+  const int C = (v.max_sys_atoms + kReduceChunk - 1) / kReduceChunk;
+  PDGPU_LAUNCH(k_kinetic_record, dim3(C, v.n_sys), kKinThreads, 0, st, v, k.J2kcal * k.Na, C);
 }
 void launch_vel_init_impl(const PackView &v, cudaStream_t st, double temp, const unsigned long long *seeds) {
   const Consts &k = consts();
