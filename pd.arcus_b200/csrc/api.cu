@@ -2401,8 +2401,9 @@ int pdgpu_profile_eval(pdgpu_ctx *c, int32_t sys, int32_t reps, double *ms, int6
   }
   cudaError_t ce = profile_eval_tiles(P.v, c->st, reps, ms);
   if (ce != cudaSuccess) return cuda_fail(ce, "profile_eval");
-  if ((r = sync_check(c, "profile_eval"))) return r;
-  if ((r = barrier_check(c, P))) return r;
+  int flags[F_COUNT];  // (the last of the timed forms has the grid barriers, whatever the pack's own form)
+  if ((r = small_out(c, flags, P.v.flags, sizeof flags, "profile_eval"))) return r;
+  if ((r = barrier_check(c, P, flags))) return r;
   if (counts) {
     // the still list a Born phase makes (an evaluation's chain phase
     // clears it, so it is counted after a Born phase alone)
