@@ -766,22 +766,35 @@ static int state_in(pdgpu_ctx *c, Pack &P, const double *xyz, const double *vel)
   return sync_check(c, xyz ? "set_positions" : "set_velocities");
 }
 // [n][3] out of the device: `form` enqueues the kernel that writes the
-// interleaved block to where it is given.
+// interleaved block of n atoms from i0 on to where it is given.  Without device
+// memory for the staging array (a batch may come here first, its positions
+// never having been set) the block goes in pieces through the page-locked one.
 template <typename Form>
 static int block_out(pdgpu_ctx *c, Pack &P, double *user, const char *what, Form form) {
-  const size_t bytes = sizeof(double) * 3 * (size_t)P.v.n_atoms;
-  if (double *pin = pinned(c, user, bytes)) {
-    form(pin);
+  const int N = P.v.n_atoms;
+  const size_t atom = 3 * sizeof(double), bytes = atom * (size_t)N;
+  const int most = (int)(pdgpu_ctx::kPinBytes / atom);
+  if (!pinned(c, user, bytes)) {
+    int r = pack_ensure_stage(&P);
+    if (!r) {
+      form(P.stage, 0, N);
+      PDGPU_CUDA(cudaMemcpyAsync(user, P.stage, bytes, cudaMemcpyDeviceToHost, c->st));
+      return sync_check(c, what);
+    }
+    if (!pinned(c, user, 0)) return r;
+  }
+  for (int i0 = 0; i0 < N; i0 += most) {
+    const int n = std::min(most, N - i0);
+    form((double *)c->pin, i0, n);
     int r = sync_check(c, what);
     if (r) return r;
-    memcpy(user, pin, bytes);
-    return PDGPU_OK;
+    memcpy(user + 3 * (size_t)i0, c->pin, atom * n);
   }
-  int r = pack_ensure_stage(&P);
-  if (r) return r;
-  form(P.stage);
-  PDGPU_CUDA(cudaMemcpyAsync(user, P.stage, bytes, cudaMemcpyDeviceToHost, c->st));
-  return sync_check(c, what);
+  return PDGPU_OK;
+}
+// [n][3] from three arrays, for block_out.
+static auto from_soa(pdgpu_ctx *c, const double *X, const double *Y, const double *Z) {
+  return [=](double *to, int i0, int n) { launch_soa_to_aos(to, X + i0, Y + i0, Z + i0, n, c->st); };
 }
 // A few bytes of device memory read by the host.
 static int small_out(pdgpu_ctx *c, void *dst, const void *src, size_t bytes, const char *what) {
@@ -811,8 +824,7 @@ int pdgpu_get_positions(pdgpu_ctx *c, int32_t sys, double *xyz) {
     return PDGPU_ERR_ARG;
   }
   const PackView &v = e->pack->v;
-  return block_out(c, *e->pack, xyz, "get_positions",
-                   [&](double *to) { launch_soa_to_aos(to, v.x, v.y, v.z, v.n_atoms, c->st); });
+  return block_out(c, *e->pack, xyz, "get_positions", from_soa(c, v.x, v.y, v.z));
 }
 int pdgpu_set_velocities(pdgpu_ctx *c, int32_t sys, const double *v) {
   CHECK_CTX(c);
@@ -831,8 +843,7 @@ int pdgpu_get_velocities(pdgpu_ctx *c, int32_t sys, double *v) {
     return PDGPU_ERR_ARG;
   }
   const PackView &w = e->pack->v;
-  return block_out(c, *e->pack, v, "get_velocities",
-                   [&](double *to) { launch_soa_to_aos(to, w.vx, w.vy, w.vz, w.n_atoms, c->st); });
+  return block_out(c, *e->pack, v, "get_velocities", from_soa(c, w.vx, w.vy, w.vz));
 }
 
 int pdgpu_get_forces(pdgpu_ctx *c, int32_t sys, double *f) {
@@ -843,8 +854,9 @@ int pdgpu_get_forces(pdgpu_ctx *c, int32_t sys, double *f) {
     return PDGPU_ERR_ARG;
   }
   Pack &P = *e->pack;
-  return block_out(c, P, f, "get_forces",
-                   [&](double *to) { launch_forces_out(P.v, consts().N_per_kcalmolA, to, c->st); });
+  return block_out(c, P, f, "get_forces", [&](double *to, int i0, int n) {
+    launch_forces_out(P.v, consts().N_per_kcalmolA, to, i0, n, c->st);
+  });
 }
 
 int pdgpu_get_born_radii(pdgpu_ctx *c, int32_t sys, double *born) {
@@ -1360,13 +1372,8 @@ int pdgpu_sasa_lcpo_get(pdgpu_ctx *c, int32_t sys, double *sasa, double *deriv) 
     return PDGPU_OK;
   }
   if (sasa) PDGPU_CUDA(cudaMemcpyAsync(sasa, lc.sasa, sizeof(double) * N, cudaMemcpyDeviceToHost, c->st));
-  if (deriv) {  // interleaved on the device, one block copied
-    int r = pack_ensure_stage(&P);
-    if (r) return r;
-    launch_soa_to_aos(P.stage, lc.deriv, lc.deriv + N, lc.deriv + 2 * N, (int)N, c->st);
-    PDGPU_CUDA(cudaMemcpyAsync(deriv, P.stage, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, c->st));
-  }
-  return sync_check(c, "sasa_lcpo_get");
+  if (!deriv) return sync_check(c, "sasa_lcpo_get");
+  return block_out(c, P, deriv, "sasa_lcpo_get", from_soa(c, lc.deriv, lc.deriv + N, lc.deriv + 2 * N));
 }
 }  // extern "C"
 

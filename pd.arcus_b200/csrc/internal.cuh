@@ -396,8 +396,8 @@ void launch_pack_positions(const PackView &v, cudaStream_t st);
 void launch_state_in(const PackView &v, const double *X, const double *V, cudaStream_t st);
 void launch_state_out(const PackView &v, double *X, double *V, cudaStream_t st);
 void launch_soa_to_aos(double *aos, const double *X, const double *Y, const double *Z, int n, cudaStream_t st);
-// forces in N, interleaved [n][3], for the caller (scale: kcal/mol/A -> N)
-void launch_forces_out(const PackView &v, double scale, double *out, cudaStream_t st);
+// forces in N of n atoms from i0 on, interleaved [n][3], for the caller (scale: kcal/mol/A -> N)
+void launch_forces_out(const PackView &v, double scale, double *out, int i0, int n, cudaStream_t st);
 void launch_zero(const PackView &v, cudaStream_t st);
 void launch_zero_bonded(const PackView &v, cudaStream_t st);
 // neighbour list: build phases.  count -> (host may read total) -> fill

@@ -77,10 +77,10 @@ __global__ void k_soa_to_aos(double *aos, const double *X, const double *Y, cons
 // this from nine pageable copies (100 us a call at 133 atoms, 437 at 20,566,
 // 20.6 ms at 568,384; with the one block 20 us, 59 us and 1.7 ms, most of it
 // the copy into the caller's pageable buffer).
-__global__ void k_forces_out(PackView v, double scale, double *out) {
+__global__ void k_forces_out(PackView v, double scale, double *out, int i0, int n) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * v.n_atoms) return;
-  const int i = t / 3, k = t - 3 * i;
+  if (t >= 3 * n) return;
+  const int i = i0 + t / 3, k = t % 3;
   const long long *f = k == 0 ? v.fx : (k == 1 ? v.fy : v.fz);
   const double *g = k == 0 ? v.gx : (k == 1 ? v.gy : v.gz);
   const long long *h = k == 0 ? v.hx : (k == 1 ? v.hy : v.hz);
@@ -88,8 +88,8 @@ __global__ void k_forces_out(PackView v, double scale, double *out) {
                              __dmul_rn((double)h[i], kInvJScale));
   out[t] = __dmul_rn(s, scale);
 }
-void launch_forces_out(const PackView &v, double scale, double *out, cudaStream_t st) {
-  if (v.n_atoms) PDGPU_LAUNCH(k_forces_out, (3 * v.n_atoms + 255) / 256, 256, 0, st, v, scale, out);
+void launch_forces_out(const PackView &v, double scale, double *out, int i0, int n, cudaStream_t st) {
+  if (n > 0) PDGPU_LAUNCH(k_forces_out, (3 * n + 255) / 256, 256, 0, st, v, scale, out, i0, n);
 }
 
 // The state from / to interleaved [n][3] blocks in one launch: positions (with

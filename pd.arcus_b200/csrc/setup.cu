@@ -340,6 +340,7 @@ int pack_upload_lcpo(Pack *p, const std::vector<const SystemHost *> &systems) {
 int pack_ensure_stage(Pack *p) {
   if (p->stage) return PDGPU_OK;
   if (palloc(p, &p->stage, 3 * (size_t)p->v.n_atoms) != cudaSuccess || cudaStreamSynchronize(p->st) != cudaSuccess) {
+    cudaGetLastError();  // (not the next call's error)
     set_error("device allocation failed (state staging)");
     return PDGPU_ERR_NOMEM;
   }
