@@ -119,7 +119,7 @@ int entry_materialize(int device, SysEntry *e, bool sync) {
     return PDGPU_ERR_NOMEM;
   }
   e->pack.reset(p);
-  if (xalloc(e, &e->seeds, e->nsys()) != cudaSuccess || xalloc(e, &e->step_dev, 3) != cudaSuccess) {
+  if (xalloc(e, &e->seeds, e->nsys()) != cudaSuccess || xalloc(e, &e->step_dev, SD_COUNT) != cudaSuccess) {
     set_error("device allocation failed");
     return PDGPU_ERR_NOMEM;
   }
@@ -1639,7 +1639,9 @@ void pdgpu::md_step_enqueue(cudaStream_t st, SysEntry *e, const MDCoef &k, int q
   // reads: that record must be done
   P.wait_energy(st, b ^ 1);
   P.wait_energy(st, b);
-  launch_md_step_impl(P.v, st, k, nullptr, e->step_dev, P.is_h, e->seeds, e->traj_dev, e->traj_every,
+  MDCoef kq = k;
+  kq.step = q;
+  launch_md_step_impl(P.v, st, kq, nullptr, e->step_dev, P.is_h, e->seeds, e->traj_dev, e->traj_every,
                       e->traj_dev_cap);
   // the step's energy record beside the next step's evaluation
   if (record_apart(P) && behind_first_phase(P, P.coop_md)) {
@@ -1818,17 +1820,17 @@ static int md_run_impl(pdgpu_ctx *c, SysEntry *e, const pdgpu_md_params *p, int3
   // (EM_GATE), so the state is the failed block's.  Not with trajectory
   // frames (each block's are copied before the next writes the ring) nor with the
   // cooperative launch (its barrier's counters are mended between blocks).
-  if (!e->pin_flags && cudaHostAlloc((void **)&e->pin_flags, sizeof(int) * (2 * F_COUNT + 3), 0) != cudaSuccess) {
+  if (!e->pin_flags && cudaHostAlloc((void **)&e->pin_flags, sizeof(int) * (2 * F_COUNT + SD_COUNT), 0) != cudaSuccess) {
     e->pin_flags = nullptr;
     set_error("page-locked host allocation failed (MD flags)");
     return PDGPU_ERR_NOMEM;
   }
   for (cudaEvent_t &ev : e->block_ev)
     if (!ev) PDGPU_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-  int *steps0 = e->pin_flags + 2 * F_COUNT;  // step counter, first step, finished-system count
-  steps0[0] = steps0[1] = first_step;
-  steps0[2] = 0;
-  PDGPU_CUDA(cudaMemcpyAsync(e->step_dev, steps0, sizeof(int) * 3, cudaMemcpyHostToDevice, c->st));
+  int *steps0 = e->pin_flags + 2 * F_COUNT;
+  steps0[SD_STEP] = steps0[SD_BLOCK] = steps0[SD_FIRST] = first_step;
+  steps0[SD_DONE] = 0;
+  PDGPU_CUDA(cudaMemcpyAsync(e->step_dev, steps0, sizeof(int) * SD_COUNT, cudaMemcpyHostToDevice, c->st));
   cudaEventRecord(P.ev0, c->st);
   // One block of the run's steps from s, enqueued with its flag copy, and the
   // host's notes on what it leaves on the device.
@@ -1984,8 +1986,8 @@ static int md_run_impl(pdgpu_ctx *c, SysEntry *e, const pdgpu_md_params *p, int3
         return PDGPU_ERR_STATE;
       }
       PDGPU_CUDA(cudaMemsetAsync(v.flags + F_NL_OVERFLOW, 0, sizeof(int), c->st));
-      steps0[0] = first_step + done;
-      PDGPU_CUDA(cudaMemcpyAsync(e->step_dev, steps0, sizeof(int), cudaMemcpyHostToDevice, c->st));
+      steps0[SD_STEP] = steps0[SD_BLOCK] = first_step + done;
+      PDGPU_CUDA(cudaMemcpyAsync(e->step_dev, steps0, sizeof(int) * 2, cudaMemcpyHostToDevice, c->st));
       enqueued = done;
       nrun = 0;
       continue;

@@ -51,8 +51,7 @@ __device__ __forceinline__ double chunk_sum(const double *p, int b, int e) {
   return t;
 }
 
-// hist: [step][sys][3] (epot, ekin, etot); step_dev[0] current step,
-// step_dev[1] first step of the run, step_dev[2] finished-system counter.
+// hist: [step][sys][3] (epot, ekin, etot); step_dev: StepSlot.
 __global__ void __launch_bounds__(kEnergyThreads) k_energy(PackView v, int mode, int C, double J2kcalmol,
                                                            double *hist, int *step_dev, MinCtl ctl) {
   // the ranges are fixed with the pack: read before the wait
@@ -93,7 +92,7 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energy(PackView v, int mode,
   if (warp == kEnergyWarps - 1) {
     if (lane < E_COUNT) sE[lane] = __ldcg(E + lane);
     if (lane == 30) sflag = __ldcg(sflags + s);
-    if (lane == 31 && (mode & EM_RECORD)) sk = __ldcg(step_dev) - __ldcg(step_dev + 1);
+    if (lane == 31 && (mode & EM_RECORD)) sk = __ldcg(step_dev + SD_STEP) - __ldcg(step_dev + SD_FIRST);
   }
   if (pair) {
     sh[P_VDW][x] = chunk_sum(ep + (size_t)AE_VDW * N, lo[0], hi[0]);
@@ -220,16 +219,19 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energy(PackView v, int mode,
       h[lane] = sE[lane == 0 ? E_EPOT : lane == 1 ? E_EKIN : E_ETOT];
     }
     // the last system to finish advances the step (every block has read
-    // step_dev[0] before it counts itself finished)
+    // SD_STEP before it counts itself finished)
     if ((mode & EM_RECORD) && lane == 0) {
       __threadfence();
-      int done = atomicAdd(&step_dev[2], 1);
+      int done = atomicAdd(&step_dev[SD_DONE], 1);
       if (done == v.n_sys - 1) {
-        step_dev[2] = 0;
-        if ((mode & EM_GATE) && (__ldcg(&v.flags[F_NAN]) || __ldcg(&v.flags[F_LCPO_CAND])))
-          atomicExch(&v.flags[F_NL_OVERFLOW], kGateShut);
+        step_dev[SD_DONE] = 0;
+        if (mode & EM_GATE) {
+          step_dev[SD_BLOCK] = __ldcg(step_dev + SD_STEP) + 1;
+          if (__ldcg(&v.flags[F_NAN]) || __ldcg(&v.flags[F_LCPO_CAND]))
+            atomicExch(&v.flags[F_NL_OVERFLOW], kGateShut);
+        }
         __threadfence();
-        atomicAdd(&step_dev[0], 1);
+        atomicAdd(&step_dev[SD_STEP], 1);
       }
     }
   }

@@ -29,16 +29,18 @@ namespace pdgpu {
 // e_atom[AE_KIN] and is reduced per system afterwards.
 // The thermostat's normals depend on the step, the atom and its system's key
 // only, so they are drawn before the wait for the force passes (under a
-// programmatic dependent launch, beside the last pass's tail).  The step
-// counter is final by then: the step's launch waits on the event of the
-// energy record that advanced it, a full dependency.  The atom's mass,
-// velocity and position (the previous step's, complete before this step's
-// first phase passed its own wait) and the noise widths of its mass are ready
-// before the wait too; after it come the nine force loads and the update.
+// programmatic dependent launch, beside the last pass's tail).  The step is the
+// block's first one, which stays while the block runs, and the number of this
+// launch in it: the counter itself is advanced by the previous step's record,
+// which may still run (in a graph every edge into this launch is programmatic,
+// the one from that record too).  The atom's mass, velocity and position (the
+// previous step's, complete before this step's first phase passed its own
+// wait) and the noise widths of its mass are ready before the wait too; after
+// it come the nine force loads and the update.
 __global__ void k_md_step(PackView v, MDDev d, const double *normals, const int *step_dev) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = i < v.n_atoms;
-  const int step = !live ? 0 : step_dev ? *step_dev : d.c.step;
+  const int step = !live ? 0 : step_dev ? step_dev[SD_BLOCK] + d.c.step : d.c.step;
   double nr[6];
   const bool pre = live && !normals && md_draws_normals(v, d, step, i);
   MDIn in;

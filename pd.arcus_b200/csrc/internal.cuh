@@ -90,7 +90,8 @@ enum EnergyMode {
   EM_BONDED = 8,       // bond, angle, torsion, bond virial
   EM_KINETIC = 16,     // ekin, etot
   EM_RECORD = 32,      // history row + step counter advance (step loops)
-  EM_GATE = 512,       // with EM_RECORD: F_NL_OVERFLOW = kGateShut after a NaN or F_LCPO_CAND (the next block skips)
+  EM_GATE = 512,       // with EM_RECORD, a block's last: the next block's SD_BLOCK, and
+                       // F_NL_OVERFLOW = kGateShut after a NaN or F_LCPO_CAND (that block skips)
   EM_ASSIGN = 64,      // form the record from zero (its slots were not zeroed before the step)
   EM_SURF = 128,       // LCPO surface term: epot_surf
   EM_PAIR_GB_SLOW = 256  // GB with FastMode off (calcBornForces): pol + self added to epot alone;
@@ -127,6 +128,12 @@ struct StepSrc {
   int stride = 0;
   int imm = 0;
 };
+
+// An MD run's step counters on the device (ints).  The records advance
+// SD_STEP; SD_BLOCK, the step a block of steps began with, stays while the
+// block runs, so the integrators can read it before anything of their own
+// step is complete.
+enum StepSlot { SD_STEP = 0, SD_BLOCK, SD_FIRST, SD_DONE, SD_COUNT };  // ... the run's first step, finished systems
 
 // A minimiser step's control, taken where its energy is formed (minstep.cuh).
 struct MinState;
@@ -481,7 +488,7 @@ struct MDCoef {
   // per-step constants of the Langevin update, formed once on the host:
   // (1 - c0/c1)/(gamma dt), c0 c2 / c1, 1/gamma, sqrt(1 - crv^2)
   double kick1, c0c2_c1, inv_gamma, sq_crv;
-  int integrator, step, steps, use_normals, stochastic_h;
+  int integrator, step, steps, use_normals, stochastic_h;  // step: from SD_BLOCK on where there are counters
   unsigned long long seed;
 };
 void launch_md_step(const PackView &v, cudaStream_t st, const MDCoef &c, const double *normals,

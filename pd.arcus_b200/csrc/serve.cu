@@ -83,8 +83,7 @@ constexpr double kAgeMs = 1000.0;  // least-work admission: a job queued this lo
 struct PinHead {
   long long total;     // list entries after a count pass
   int flags[F_COUNT];  // device flags (overflow, NaN)
-  int step;            // MD: step of the block start (host -> device)
-  int pad;
+  int step[2];         // MD: SD_STEP and SD_BLOCK at the block's start (host -> device)
 };
 
 struct Job {
@@ -339,12 +338,12 @@ void pdgpu_server::enqueue_md_block(Job *j) {
   if (rebuild && every > 1) block = std::min(every, steps - j->md_done);
   bool use_graph = p.UseGraph && rebuild && block == every && every > 1;
   j->block = block;
-  j->pin->step = j->md_done;
+  j->pin->step[SD_STEP] = j->pin->step[SD_BLOCK] = j->md_done;
   cudaMemsetAsync(v.flags + F_NL_OVERFLOW, 0, sizeof(int), j->st);
   // a group goes on past a member's NaN energy (the member is marked failed
   // from its energy history at the end)
   if (!j->group.empty()) cudaMemsetAsync(v.flags + F_NAN, 0, sizeof(int), j->st);
-  cudaMemcpyAsync(e->step_dev, &j->pin->step, sizeof(int), cudaMemcpyHostToDevice, j->st);
+  cudaMemcpyAsync(e->step_dev, j->pin->step, sizeof j->pin->step, cudaMemcpyHostToDevice, j->st);
   if (use_graph) {
     if (!e->gexec || e->gkey != "md") {
       e->drop_graph();
@@ -555,7 +554,7 @@ void pdgpu_server::admit(Job *j, const std::vector<Job *> &more) {
       return;
     }
     e->hist_cap = j->spec.steps;
-    j->pin->step = 0;
+    j->pin->step[SD_STEP] = j->pin->step[SD_BLOCK] = 0;
     // every member's seed, staged through the pinned block (the minimiser
     // state's room, which an MD job does not use)
     static_assert(sizeof(unsigned long long) <= 8, "seed size");
