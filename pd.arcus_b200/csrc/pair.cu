@@ -154,13 +154,15 @@ void launch_soa_to_aos(double *aos, const double *X, const double *Y, const doub
 // the forces of a step that does nothing (the flag): they are what the caller
 // of a failed run reads.
 __global__ void k_zero_bonded(PackView v) {
-  PDGPU_DEP_ENTRY();
   if (v.flags[F_NL_OVERFLOW]) return;
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < 3 * (size_t)v.n_atoms) v.fx[i] = 0;
+  const size_t i = 2 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x), n = 3 * (size_t)v.n_atoms;
+  if (i + 1 < n)
+    *reinterpret_cast<longlong2 *>(v.fx + i) = make_longlong2(0, 0);  // (a pool allocation: 256-byte aligned)
+  else if (i < n)
+    v.fx[i] = 0;
 }
 void launch_zero_bonded(const PackView &v, cudaStream_t st) {
-  if (v.n_atoms) PDGPU_LAUNCH_DEP(k_zero_bonded, (3 * (size_t)v.n_atoms + 255) / 256, 256, 0, st, v);
+  if (v.n_atoms) PDGPU_LAUNCH(k_zero_bonded, (3 * (size_t)v.n_atoms + 511) / 512, 256, 0, st, v);
 }
 
 __global__ void k_zero(PackView v) {
