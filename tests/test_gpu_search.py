@@ -48,3 +48,40 @@ def test_search_capacities(side, spacing, order, special, gpu_ctx):
     c = _counts(ws)
     assert c[3] == c[2] // 2 and c[4] > 0
     ws.close()
+
+
+def test_search_capacities_with_finite_energies(gpu_ctx):
+    """The large shuffled system again at a spacing where no pair overlaps so
+    far that its energy is not finite: a lost tile, or bond-order rows given to
+    the wrong tile, then show in the energies too."""
+    rng = np.random.default_rng(5)
+    g = np.arange(21)
+    pos = 3.4 * np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3).astype(np.float64)
+    pos = (pos + rng.normal(0.0, 0.1, pos.shape))[rng.permutation(21 ** 3)]
+    n = len(pos)
+    arrays, meta = _system(pos, np.arange(n) % 300)
+    partners = [[] for _ in range(n)]
+    # 60 pairs inside the cutoff, each in a tile of its own
+    dist = np.linalg.norm(pos[:32, None] - pos[None], axis=2)
+    near = dist.argmin(axis=0)
+    close = [j for j in range(32, n) if 4.0 < dist[near[j], j] < 12.0]
+    for j in {j // 8: j for j in close[::-1]}.values():
+        if sum(len(p) for p in partners) < 120:
+            partners[near[j]].append(int(j))
+            partners[j].append(int(near[j]))
+    arrays["cov14_ptr"] = np.cumsum([0] + [len(p) for p in partners]).astype(np.int32)
+    arrays["cov14_idx"] = np.array([j for p in partners for j in sorted(p)], dtype=np.int32)
+    ws, ff = build_workspace(arrays, meta, gpu_ctx)
+    ws.setPairPath(0)
+    ws.nlist().calcNewList()
+    ptr, data = ws.nlist().getData(shadow=True)
+    special = (np.asarray(data[:ptr[32]]) >> 24) < 7
+    assert special.sum() > 24 and np.diff(ptr[:33]).sum() > 256 * 8
+    ws.setPairPath(1)
+    listed = _forces_energies(ws, ff)
+    ws.nlist().calcNewList()
+    searched = _forces_energies(ws, ff)
+    for a, b in zip(searched, listed):
+        assert np.all(np.isfinite(np.asarray(a)))
+        np.testing.assert_array_equal(a, b)
+    ws.close()
