@@ -1817,7 +1817,8 @@ static int md_run_impl(pdgpu_ctx *c, SysEntry *e, const pdgpu_md_params *p, int3
   // atoms, 19.0 -> 18.5 at 985, 20.9 -> 20.2 at 1,662, 55.4 -> 54.6 at 20,566).
   // A block enqueued behind one that failed does nothing: an overflow's flag is
   // still set, and after a NaN or a full overlap list the last record sets it
-  // (EM_GATE), so the state is the failed block's.  Not with trajectory
+  // (EM_GATE), so the state is the failed block's, its pair structure (the
+  // rebuild looks at the flag too) and forces included.  Not with trajectory
   // frames (each block's are copied before the next writes the ring) nor with the
   // cooperative launch (its barrier's counters are mended between blocks).
   if (!e->pin_flags && cudaHostAlloc((void **)&e->pin_flags, sizeof(int) * (2 * F_COUNT + SD_COUNT), 0) != cudaSuccess) {

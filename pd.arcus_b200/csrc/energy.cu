@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energy(PackView v, int mode,
   }
   if (mine > 1) {
     // the last block of this system to finish forms the record: warp w adds
-    // slots w and w + 8 over the chunks, lane l the chunks l, l + 32, ...
+    // slot w (of P_COUNT) over the chunks, lane l the chunks l, l + 32, ...
     // (loads in parallel), then a fixed shuffle tree
     __threadfence();
     __syncthreads();

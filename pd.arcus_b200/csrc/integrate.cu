@@ -153,7 +153,7 @@ __global__ void k_vel_scale(PackView v, double kB, double temp, double kcal2J_pe
 // last block takes the step's decision (min_control).  An atom per thread: a
 // step waits for this launch and its blocks for twelve loads an atom, which
 // the record's 4,096-item chunks made sixteen times in a row.  A step's share
-// (CG step minus SD step), 4,096 items -> 256: 506 atoms 7.2 -> 4.0 us, 2,972
+// (CG step minus SD step), 4,096 items -> 256: 985 atoms 7.2 -> 4.0 us, 2,972
 // 14.2 -> 3.6, 20,566 17.2 -> 5.5.  A system of one chunk needs no second stage.
 constexpr int kDotChunk = 256;
 static_assert(2 * (kReduceChunk / kDotChunk) <= kPartSlots, "two partials a chunk fit the reduction buffer");

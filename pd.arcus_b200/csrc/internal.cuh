@@ -562,14 +562,24 @@ long long end_capture_count();
 
 // Programmatic dependent launch for the kernels of the evaluation and step
 // chain.  A kernel launched with PDGPU_LAUNCH_DEP may be scheduled while the
-// kernel before it in the stream still runs; it must begin with
-// PDGPU_DEP_ENTRY(), which waits until every earlier kernel of the stream
-// has completed and its memory is visible (griddepcontrol.wait) before the
-// kernel touches global memory, then lets the next kernel be scheduled in
-// turn (griddepcontrol.launch_dependents).  The launch of kernel k+1 thus
-// overlaps the run of kernel k; no kernel reads or writes anything before
-// its predecessors are done.  PDGPU_PDL=0 in the environment turns the
-// overlap off (plain launches).
+// kernels it depends on still run.  PDGPU_DEP_ENTRY() waits until these have
+// completed and their memory is visible (griddepcontrol.wait), then lets the
+// next kernel be scheduled in turn (griddepcontrol.launch_dependents), so the
+// launch of kernel k+1 overlaps the run of kernel k.  The rules:
+// - No kernel writes before its wait, and what it reads there (k_md_step,
+//   k_min_update, k_min_dots, k_energy, k_tile_search and the phases of
+//   k_eval_tiles read some) was complete before the kernels it depends on
+//   passed their own waits: the results of these themselves are not, those of
+//   the kernels before them are.
+// - That holds because no block triggers before its own wait, and of every
+//   launch some block waits: blocks without work may leave at once (past the
+//   active ones of k_eval_tiles), block 0 does not.  Under the overflow flag
+//   whole launches leave at once; what follows them in the block writes
+//   nothing then.
+// - In a captured graph EVERY edge from a kernel into such a launch is a
+//   programmatic one, also that of an event of another stream: an event is
+//   no reason to read something before the wait.
+// PDGPU_PDL=0 in the environment turns the overlap off (plain launches).
 #define PDGPU_DEP_ENTRY()                                          \
   do {                                                             \
     asm volatile("griddepcontrol.wait;" ::: "memory");             \
