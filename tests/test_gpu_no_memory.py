@@ -27,6 +27,10 @@ class _Full:
         for p in self.held:
             self.cu.cuMemFreeAsync(ctypes.c_uint64(p), None)
         assert self.cu.cuStreamSynchronize(None) == 0
+        dev, pool = ctypes.c_int(0), ctypes.c_void_p()  # and out of the pool, which keeps what it has
+        assert self.cu.cuDeviceGet(ctypes.byref(dev), 0) == 0
+        assert self.cu.cuDeviceGetDefaultMemPool(ctypes.byref(pool), dev) == 0
+        assert self.cu.cuMemPoolTrimTo(pool, ctypes.c_size_t(0)) == 0
 
 
 def test_state_out_without_staging_memory(gpu_ctx):
